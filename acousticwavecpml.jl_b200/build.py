@@ -17,8 +17,9 @@ ROOT = os.path.dirname(HERE)
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 SOURCES = ["csrc/awc_api.cu", "csrc/awc_adjoint.cu", "csrc/awc_batch.cu", "csrc/awc_learned.cu",
-           "csrc/awc_static.cu", "csrc/awc_tb.cu"]
-HEADERS = ["csrc/awc_kernels.cuh", "csrc/awc_tb.cuh", "csrc/awc_ctx.h", "../include/awcpml.h"]
+           "csrc/awc_loop2d.cu", "csrc/awc_static.cu", "csrc/awc_tb.cu"]
+HEADERS = ["csrc/awc_kernels.cuh", "csrc/awc_loop2d.cuh", "csrc/awc_loop2d.h", "csrc/awc_tb.cuh",
+           "csrc/awc_ctx.h", "../include/awcpml.h"]
 OUT = os.path.join(HERE, "lib", "libawcpml.so")
 OBJ = os.path.join(HERE, "lib", "obj")
 FLAGS = [*ARCH, "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall"]

@@ -27,6 +27,7 @@
 #include "../../include/awcpml.h"
 #include "awc_ctx.h"
 #include "awc_kernels.cuh"
+#include "awc_loop2d.h"
 #include "awc_tb.cuh"
 
 namespace {
@@ -303,6 +304,11 @@ struct awc_plan {
   int32_t tb_maps_rows = 0;  // rows the tensor maps were encoded for
   int32_t wait_rounds = 4096, wait_ns = 1000000, withhold = -1;
   bool is1d = false;  // a 1D problem lifted to three rows (see Lifted)
+  // 2D: the on-chip time loop (awc_loop2d.cuh), when the grid fits it
+  awc::Loop2D loop;
+  int32_t loop_fits = -1;    // -1 not looked at since the model was uploaded
+  bool loop_ready = false;   // its lists match the current shot
+  std::vector<int32_t> h_rec_off, h_rec_ids;  // receiver groups (host copy)
   // run state
   int64_t step = 0;
   StepState state;
@@ -575,7 +581,9 @@ int plan_upload(awc_plan* P, const double* vel, const double* coeffs, const int6
       }
     }
     if (p->ndim == 3) make_regions(P);
+    P->loop_fits = -1;
   }
+  P->loop_ready = false;
   P->tb_io_shape = ~0ull;
   // every node carrying sources and/or receivers, in first-appearance order
   // (sources first); its sources are summed in source order
@@ -620,6 +628,8 @@ int plan_upload(awc_plan* P, const double* vel, const double* coeffs, const int6
     std::vector<int32_t> soff, sids, roff, rids;
     csr(sg, soff, sids);
     csr(rg, roff, rids);
+    P->h_rec_off = roff;
+    P->h_rec_ids = rids;
     CUDA_TRY(err, cudaMemcpyAsync(P->src_off, soff.data(), soff.size() * 4, cudaMemcpyHostToDevice, st));
     CUDA_TRY(err, cudaMemcpyAsync(P->rec_off, roff.data(), roff.size() * 4, cudaMemcpyHostToDevice, st));
     if (!sids.empty())
@@ -1297,6 +1307,74 @@ int launch_pass2(awc_plan* P, int64_t it, const StepState& stt, cudaStream_t st)
 // Whether the launch sequence of this plan advances two steps per pass.
 bool two_step(const awc_plan* P) { return P->depth == 2 && !P->keep; }
 
+awc::LoopShotHost loop_shot(const awc_plan* P) {
+  const awc_problem* p = &P->p;
+  awc::LoopShotHost H;
+  H.nx = p->nx;
+  H.ny = p->ny;
+  H.px = P->px;
+  H.halo = p->halo;
+  const double d[2] = {p->dx, p->dy};
+  for (int a = 0; a < 2; ++a) {
+    H.inv_d[a] = 1.0 / d[a];
+    H.inv_d2[a] = 1.0 / (d[a] * d[a]);
+    for (int s = 0; s < 2; ++s) {
+      H.active[a][s] = P->active[a][s];
+      for (int q = 0; q < 2; ++q) H.psi[a][s][q] = P->psi[a][s][q];
+      H.xi[a][s] = P->xi[a][s];
+    }
+  }
+  if (P->is1d) H.inv_d[1] = H.inv_d2[1] = 0.0;  // no y derivative on the line
+  for (int b = 0; b < 3; ++b) H.buf[b] = P->buf[b];
+  H.fact = P->fact;
+  H.coef = P->coef;
+  H.src_off = P->src_off;
+  H.src_ids = P->src_ids;
+  H.stf = P->stf;
+  H.traces = P->traces;
+  H.nsrc = (int32_t)p->nsrc;
+  H.nrec = (int32_t)p->nrec;
+  H.nodes = &P->io_nodes;
+  H.rec_off = &P->h_rec_off;
+  H.rec_ids = &P->h_rec_ids;
+  return H;
+}
+
+// Whether a run of n steps goes through the on-chip loop: a 2D grid that fits
+// it, for long enough, its kept fields (if any) evenly spaced in memory.
+bool use_loop(awc_plan* P, int64_t n) {
+  if (P->p.ndim != 2 || n < awc::kLoopMinSteps) return false;
+  if (P->loop_fits < 0)
+    P->loop_fits = P->loop.fits(P->ctx, P->p.precision == AWC_F64, {loop_shot(P)}) ? 1 : 0;
+  if (!P->loop_fits) return false;
+  for (int64_t m = 2; m < P->keep_count; ++m)
+    if ((char*)P->keep[m] - (char*)P->keep[m - 1] != (char*)P->keep[1] - (char*)P->keep[0])
+      return false;
+  return true;
+}
+
+// n steps from `start` in one launch; stt becomes the state after them.
+int loop_range(awc_plan* P, int64_t start, int64_t n, StepState& stt, cudaStream_t st) {
+  awc::LoopSpan sp;
+  sp.it0 = start;
+  sp.n = n;
+  for (int b = 0; b < 3; ++b) sp.in[b] = stt.ord[b];
+  sp.par_in = stt.psi_par;
+  // the three buffers rotate with period 3 and ψ with period 2
+  for (int64_t m = 0; m < n % 6; ++m) stt.step1();
+  for (int b = 0; b < 3; ++b) sp.out[b] = stt.ord[b];
+  sp.par_out = stt.psi_par;
+  if (P->keep && P->keep_count > 0) {
+    sp.keep = P->keep[0];
+    sp.keep_stride = P->keep_count > 1
+                         ? (int64_t)((char*)P->keep[1] - (char*)P->keep[0]) / (int64_t)P->esz
+                         : 0;
+    sp.keep_first = P->keep_first;
+    sp.keep_count = P->keep_count;
+  }
+  return P->loop.run(P->ctx, sp, st);
+}
+
 // Launches steps [start, start + n) from state `stt` (updated to the state
 // after them): two-step passes while two steps remain at depth 2, else
 // one-step launches.
@@ -1332,15 +1410,24 @@ int launch_range(awc_plan* P, int64_t start, int64_t n, StepState& stt, cudaStre
 
 // Kernel launches of n steps from the current state.
 int64_t launch_count(const awc_plan* P, int64_t n) {
+  if (use_loop(const_cast<awc_plan*>(P), n)) return 1;
   const int64_t one = (P->p.ndim == 3 && P->has_core && P->nbox > 0) ? 2 : 1;
   if (!two_step(P)) return one * n;
   const int64_t per_pass = (P->tb_ntiles[0] > 0 ? 1 : 0) + (P->tb_ntiles[1] > 0 ? 1 : 0);
   return per_pass * (n / 2) + one * (n % 2);
 }
 
-// Everything a launch sequence depends on besides the step index.
-int prepare_launch(awc_plan* P) {
+// Everything a launch sequence depends on besides the step index, for a run
+// through the on-chip loop (loop) or the per-step kernels.
+int prepare_launch(awc_plan* P, bool loop = false) {
   int rc;
+  if (loop) {
+    if (P->loop_ready) return AWC_OK;
+    if ((rc = P->loop.prepare(P->ctx, P->p.precision == AWC_F64, {loop_shot(P)}, P->err_flag)))
+      return rc;
+    P->loop_ready = true;
+    return AWC_OK;
+  }
   if ((rc = ensure_io(P))) return rc;
   if (P->p.ndim == 3 && P->has_core && (rc = ensure_maps(P))) return rc;
   if (two_step(P) && ((rc = ensure_tb(P)) || (rc = ensure_tb_maps(P)))) return rc;
@@ -1817,7 +1904,9 @@ int awc_plan_run(awc_plan* P, int64_t nsteps, int32_t use_graph, float* ms) {
   if (ms) *ms = 0.f;
   if (n <= 0) return AWC_OK;
   int rc;
-  if ((rc = prepare_launch(P))) return rc;
+  const bool loop = use_loop(P, n);  // one launch: nothing to capture
+  if (loop) use_graph = 0;
+  if ((rc = prepare_launch(P, loop))) return rc;
   cudaGraphExec_t ex = nullptr;
   if (use_graph && (rc = get_graph(P, P->step, n, &ex))) return rc;
   CUDA_TRY(&C->err, cudaEventRecord(C->ev0, C->stream));
@@ -1825,7 +1914,9 @@ int awc_plan_run(awc_plan* P, int64_t nsteps, int32_t use_graph, float* ms) {
     CUDA_TRY(&C->err, cudaGraphLaunch(ex, C->stream));
   }
   StepState end = P->state;
-  if (!use_graph) {
+  if (loop) {
+    if ((rc = loop_range(P, P->step, n, end, C->stream))) return rc;
+  } else if (!use_graph) {
     if ((rc = launch_range(P, P->step, n, end, C->stream))) return rc;
   } else {
     for (int64_t it = P->step; it < P->step + n;) {  // the state the graph leaves
@@ -1866,7 +1957,8 @@ int awc_plan_run_snapshots(awc_plan* P, int64_t nsteps, int64_t nsave, double* o
   if (count > 0 && !out) return set_err(&C->err, AWC_ERR_INVALID, "out is NULL");
   CUDA_TRY(&C->err, cudaSetDevice(C->device));
   int rc;
-  if ((rc = prepare_launch(P))) return rc;
+  const bool loop = use_loop(P, nsave);
+  if ((rc = prepare_launch(P)) || (loop && (rc = prepare_launch(P, true)))) return rc;
   // two device staging slots of N doubles: the unpitched copy of snapshot k
   // goes to slot k % 2, then to the host on the second stream while the next
   // steps run
@@ -1890,7 +1982,9 @@ int awc_plan_run_snapshots(awc_plan* P, int64_t nsteps, int64_t nsave, double* o
   const int blocks = grid_for(C, P->N, 256);
   while (it < last) {
     const int64_t next = std::min<int64_t>(last, (it / nsave + 1) * nsave);
-    if ((rc = launch_range(P, it, next - it, stt, C->stream))) {
+    rc = loop && next - it >= awc::kLoopMinSteps ? loop_range(P, it, next - it, stt, C->stream)
+                                                 : launch_range(P, it, next - it, stt, C->stream);
+    if (rc) {
       cleanup();
       return rc;
     }

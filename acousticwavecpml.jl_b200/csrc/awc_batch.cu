@@ -20,6 +20,7 @@
 #include "../../include/awcpml.h"
 #include "awc_ctx.h"
 #include "awc_kernels.cuh"
+#include "awc_loop2d.h"
 
 namespace {
 
@@ -68,6 +69,11 @@ struct awc_batch {
   int64_t step = 0;
   std::map<std::pair<int64_t, int64_t>, cudaGraphExec_t> graphs;
   uint64_t graph_key = 0;
+  // the on-chip loop (awc_loop2d.cuh), for runs whose shots all fit it unless
+  // a launch shape of the per-step kernels was chosen
+  awc::Loop2D loop;
+  bool use_loop = true, loop_ready = false;
+  std::vector<std::vector<int32_t>> h_rec_off, h_rec_ids;  // receiver groups per shot
   double* staging = nullptr;  // inside the arena (read-out)
   int64_t staging_len = 0;
 
@@ -369,6 +375,73 @@ int launch_batch_range(awc_batch* B, int64_t start, int64_t n, cudaStream_t st) 
   return AWC_OK;
 }
 
+// What the on-chip loop needs of every shot.
+std::vector<awc::LoopShotHost> loop_shots(const awc_batch* B) {
+  std::vector<awc::LoopShotHost> out;
+  for (int32_t s = 0; s < B->nshots; ++s) {
+    const awc_problem& p = B->models[B->shots[s].model];
+    const auto& M = B->sm[s];
+    awc::LoopShotHost H;
+    H.nx = p.nx;
+    H.ny = p.ny;
+    H.px = pitch32(p.nx);
+    H.halo = p.halo;
+    const double d[2] = {p.dx, p.dy};
+    for (int a = 0; a < 2; ++a) {
+      H.inv_d[a] = 1.0 / d[a];
+      H.inv_d2[a] = 1.0 / (d[a] * d[a]);
+      for (int sd = 0; sd < 2; ++sd) {
+        H.active[a][sd] = B->active[(s * 2 + a) * 2 + sd];
+        for (int q = 0; q < 2; ++q) H.psi[a][sd][q] = B->arena + M.psi[a][sd][q];
+        H.xi[a][sd] = B->arena + M.xi[a][sd];
+      }
+    }
+    for (int b = 0; b < 3; ++b) H.buf[b] = B->arena + M.buf[b];
+    H.fact = B->arena + B->m_fact[B->shots[s].model];
+    H.coef = B->arena + M.coef;
+    H.src_off = (const int32_t*)(B->arena + M.src_off);
+    H.src_ids = (const int32_t*)(B->arena + M.src_ids);
+    H.stf = B->arena + M.stf;
+    H.traces = B->arena + M.traces;
+    H.nsrc = B->shot_nsrc[s];
+    H.nrec = B->shot_nrec[s];
+    H.nodes = &B->io_nodes[s];
+    H.rec_off = &B->h_rec_off[s];
+    H.rec_ids = &B->h_rec_ids[s];
+    out.push_back(H);
+  }
+  return out;
+}
+
+// Whether a run of n steps goes through the on-chip loop.
+bool loop_run(awc_batch* B, int64_t n) {
+  return B->use_loop && n >= awc::kLoopMinSteps &&
+         (B->loop_ready || B->loop.fits(B->ctx, B->prec == AWC_F64, loop_shots(B)));
+}
+
+// n steps of every shot from `start`: each wave of shots advances all n steps
+// in one launch before the next wave starts.
+int launch_batch_loop(awc_batch* B, int64_t start, int64_t n, cudaStream_t st) {
+  if (!B->loop_ready) {
+    const int rc = B->loop.prepare(B->ctx, B->prec == AWC_F64, loop_shots(B), (int32_t*)(B->arena + B->err));
+    if (rc) return rc;
+    B->loop_ready = true;
+  }
+  awc::LoopSpan sp;
+  sp.it0 = start;
+  sp.n = n;
+  const int64_t t[2] = {start, start + n};
+  for (int e = 0; e < 2; ++e) {  // p_t, p_{t-1}, the third buffer: t + 1, t, t + 2 modulo 3
+    int32_t* o = e ? sp.out : sp.in;
+    o[0] = (int32_t)((t[e] + 1) % 3);
+    o[1] = (int32_t)(t[e] % 3);
+    o[2] = (int32_t)((t[e] + 2) % 3);
+  }
+  sp.par_in = (int32_t)(start & 1);
+  sp.par_out = (int32_t)((start + n) & 1);
+  return B->loop.run(B->ctx, sp, st);
+}
+
 int ensure_layout(awc_batch* B) {
   if (B->io_ty == B->ty) return AWC_OK;
   return B->prec == AWC_F64 ? build_layout<double>(B) : build_layout<float>(B);
@@ -551,6 +624,8 @@ int awc_batch_create(awc_ctx* C, int32_t nmodels, const awc_problem* models,
     std::vector<int32_t> soff, sids, roff, rids;
     csr(sg, soff, sids);
     csr(rg, roff, rids);
+    B->h_rec_off.push_back(roff);
+    B->h_rec_ids.push_back(rids);
     if (up(M.src_off, soff.data(), soff.size() * 4) != cudaSuccess ||
         up(M.rec_off, roff.data(), roff.size() * 4) != cudaSuccess ||
         (!sids.empty() && up(M.src_ids, sids.data(), sids.size() * 4) != cudaSuccess) ||
@@ -597,6 +672,7 @@ int awc_batch_set_launch(awc_batch* B, int32_t tile_y, int32_t blocks_per_sm) {
                      "tile_y must be 4, 8, 16, 32 or 64; blocks_per_sm in [1, 32]");
   B->ty = tile_y;
   B->bps = blocks_per_sm;
+  B->use_loop = false;
   return AWC_OK;
 }
 
@@ -616,7 +692,9 @@ int awc_batch_run(awc_batch* B, int64_t nsteps, int32_t use_graph, float* ms) {
   if (ms) *ms = 0.f;
   if (n <= 0) return AWC_OK;
   int rc;
-  if ((rc = ensure_layout(B))) return rc;
+  const bool loop = loop_run(B, n);  // a launch per wave: nothing to capture
+  if (loop) use_graph = 0;
+  if (!loop && (rc = ensure_layout(B))) return rc;
   cudaGraphExec_t ex = nullptr;
   if (use_graph) {
     const uint64_t key = (uint64_t)B->ty | ((uint64_t)B->bps << 8);
@@ -647,6 +725,8 @@ int awc_batch_run(awc_batch* B, int64_t nsteps, int32_t use_graph, float* ms) {
   BATCH_TRY(C, cudaEventRecord(C->ev0, C->stream));
   if (use_graph) {
     BATCH_TRY(C, cudaGraphLaunch(ex, C->stream));
+  } else if (loop) {
+    if ((rc = launch_batch_loop(B, B->step, n, C->stream))) return rc;
   } else if ((rc = launch_batch_range(B, B->step, n, C->stream))) {
     return rc;
   }
@@ -711,6 +791,18 @@ int awc_batch_autotune(awc_batch* B, int64_t steps, float* best_ms_per_step) {
   float best = 1e30f;
   int32_t wty = B->ty, wbps = B->bps;
   int rc;
+  // the on-chip loop, over the steps asked for plus what makes a launch's
+  // load and store of the state a small part, as in a whole run
+  float loop_per = 1e30f;
+  B->use_loop = true;
+  const int64_t nl = std::min<int64_t>(std::max<int64_t>(steps, 64), B->nt);
+  if (loop_run(B, nl))
+    for (int rep = 0; rep < 2; ++rep) {
+      float ms = 0.f;
+      if ((rc = awc_batch_reset(B)) || (rc = awc_batch_run(B, nl, 0, &ms))) return rc;
+      loop_per = std::min(loop_per, ms / (float)nl);
+    }
+  B->use_loop = false;
   for (int32_t ty : {4, 8, 16, 32, 64})
     for (int32_t bps : {4, 8, 16}) {
       B->ty = ty;
@@ -729,7 +821,8 @@ int awc_batch_autotune(awc_batch* B, int64_t steps, float* best_ms_per_step) {
     }
   B->ty = wty;
   B->bps = wbps;
-  if (best_ms_per_step) *best_ms_per_step = best;
+  B->use_loop = loop_per < best;
+  if (best_ms_per_step) *best_ms_per_step = std::min(best, loop_per);
   return awc_batch_reset(B);
 }
 
