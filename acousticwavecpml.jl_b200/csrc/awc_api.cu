@@ -192,13 +192,13 @@ int64_t node_of(const awc_problem* p, int64_t px, const int64_t* pos, int64_t cn
   return i + px * (j + p->ny * k);
 }
 
-// Pipeline depth of the 3D core kernel: S stages let the TMA loads run S-3
-// planes ahead of the plane being computed. Five stages (two planes ahead)
-// measured best with the 64 x 4 tiles the autotuner picks on large grids:
-// 131.6 us per step at 296 x 276 x 296 against 132.4 us with four stages and
-// 131.6 us with six (more stages mean larger blocks, fewer per SM).
+// Pipeline depth of the 3D core kernel: S stages let the TMA loads run S - 2
+// planes ahead of the plane being computed. Four measured best or equal with
+// autotuned tiles: 125.0 us per step at 296 x 276 x 296 in FP32 against 125.5
+// with five and 126.3 with six (more stages, fewer blocks per SM); FP64 at
+// 203 x 187 x 171: 83.9, 84.5, 84.9 us.
 template <typename T>
-constexpr int stages() { return 5; }
+constexpr int stages() { return 4; }
 
 // Where the fields and the CPML state of the current step live. ord[0] is
 // the buffer of the newest pressure field p_s, ord[1] of p_{s-1}, ord[2] of
@@ -279,6 +279,7 @@ struct awc_plan {
   awc::Box box[6] = {};
   int32_t box_blk[7] = {};
   int32_t szc = 10;  // z planes per block of the band kernel
+  bool band_wide = false;  // node pairs in its y and z slabs (set by make_regions)
   void* stf = nullptr;     // [nt][nsrc]
   void* traces = nullptr;  // [nt][nrec]
   double* staging = nullptr;
@@ -731,6 +732,14 @@ void kernel_params(const awc_plan* P, int which, awc::StepParams<T>& S) {
   S.do_rim = P->io_k[which].do_rim;
 }
 
+// Bytes of one field on the band nodes, per SM, from which the band kernel
+// pairs the nodes of its y and z slabs: below it one node per thread keeps more
+// warps in flight. Autotuned us per step without and with pairs, n^3 grids: FP32
+// 130: 17.9, 20.9; 150: 27.0, 27.8; 175: 42.7, 42.4; 200: 60.2, 57.0; 232: 83.1,
+// 78.2; FP64 101: 18.4, 19.6; 130: 45.8, 40.6; 170: 83.9, 71.9. The line lies
+// between 150 and 175 in FP32, 101 and 130 in FP64.
+constexpr int64_t BAND_WIDE_BYTES = 72000;
+
 // Splits the interior of a 3D grid into the core box (nodes outside every
 // active CPML band: x in [halo+1, nx-halo-2] when both x sides are active,
 // and so on) and up to six disjoint shell boxes covering the rest: the two
@@ -772,13 +781,21 @@ void make_regions(awc_plan* P) {
     add(1, lo[0] - 1, lo[1], hi[1], lo[2], hi[2], 1);
     add(hi[0] + 1, n[0] - 2, lo[1], hi[1], lo[2], hi[2], 1);
   }
+  const int64_t core = empty ? 0 : (hi[0] - lo[0] + 1) * (hi[1] - lo[1] + 1) * (hi[2] - lo[2] + 1);
+  const int64_t band = (n[0] - 2) * (n[1] - 2) * (n[2] - 2) - core;
+  P->band_wide = band * (int64_t)P->esz >= BAND_WIDE_BYTES * (int64_t)P->ctx->num_sms;
   box_blocks(P);
 }
 
 // Block ranges of the band kernel: box b has its W x H columns in runs of
 // BAND_NT times chunks of szc planes.
-int64_t band_col_blocks(const awc::Box& B) {
-  const int64_t ncol = (int64_t)(B.x1 - B.x0 + 1) * (B.y1 - B.y0 + 1);
+// (y and z slabs: columns of node pairs from an even x on)
+bool band_pairs(const awc_plan* P, const awc::Box& B) { return P->band_wide && (B.kind == 3 || B.kind == 7); }
+int64_t band_width(const awc_plan* P, const awc::Box& B) {
+  return band_pairs(P, B) ? ((B.x1 - (B.x0 & ~1)) >> 1) + 1 : B.x1 - B.x0 + 1;
+}
+int64_t band_col_blocks(const awc_plan* P, const awc::Box& B) {
+  const int64_t ncol = band_width(P, B) * (B.y1 - B.y0 + 1);
   return (ncol + awc::BAND_NT - 1) / awc::BAND_NT;
 }
 
@@ -786,7 +803,7 @@ void box_blocks(awc_plan* P) {
   P->box_blk[0] = 0;
   for (int b = 0; b < P->nbox; ++b) {
     const awc::Box& B = P->box[b];
-    const int64_t blocks = band_col_blocks(B) * ((B.z1 - B.z0 + P->szc) / P->szc);
+    const int64_t blocks = band_col_blocks(P, B) * ((B.z1 - B.z0 + P->szc) / P->szc);
     P->box_blk[b + 1] = (int32_t)(P->box_blk[b] + blocks);
   }
   for (int b = P->nbox; b < 6; ++b) P->box_blk[b + 1] = P->box_blk[b];
@@ -852,10 +869,12 @@ int ensure_io(awc_plan* P) {
     for (int b = 0; b < P->nbox; ++b) {
       const awc::Box& B = P->box[b];
       if (i < B.x0 || i > B.x1 || j < B.y0 || j > B.y1 || k < B.z0 || k > B.z1) continue;
-      const int64_t l = (i - B.x0) + (int64_t)(B.x1 - B.x0 + 1) * (j - B.y0);
+      const bool pair = band_pairs(P, B);
+      const int64_t c = pair ? (i - (B.x0 & ~1)) >> 1 : i - B.x0;
+      const int64_t l = c + band_width(P, B) * (j - B.y0);
       const int64_t blk = P->box_blk[b] + l / awc::BAND_NT +
-                          band_col_blocks(B) * ((k - B.z0) / P->szc);
-      const int local = (int)(l % awc::BAND_NT);
+                          band_col_blocks(P, B) * ((k - B.z0) / P->szc);
+      const int local = (int)(l % awc::BAND_NT) * (pair ? 2 : 1) + (pair ? (int)(i & 1) : 0);
       ent[1].push_back({{blk, (k << 32) | local}, make_int4(local, (int)k, e.sgrp, e.rgrp)});
       break;
     }
@@ -1186,10 +1205,10 @@ int launch_step(awc_plan* P, int64_t it, const StepState& stt, cudaStream_t st) 
       cudaStream_t sb = core ? C->stream2 : st;
       // offsets fit in int32 when every field (and so every ψ/ξ array) does
       const unsigned nb = (unsigned)P->box_blk[P->nbox];
-      if (P->NP <= (int64_t)INT32_MAX)
-        awc::step3d_band<T, int32_t><<<nb, awc::BAND_NT, 0, sb>>>(Sh);
-      else
-        awc::step3d_band<T, int64_t><<<nb, awc::BAND_NT, 0, sb>>>(Sh);
+      const bool i32 = P->NP <= (int64_t)INT32_MAX;
+      const auto kernel = P->band_wide ? (i32 ? awc::step3d_band<T, int32_t, true> : awc::step3d_band<T, int64_t, true>)
+                                       : (i32 ? awc::step3d_band<T, int32_t, false> : awc::step3d_band<T, int64_t, false>);
+      kernel<<<nb, awc::BAND_NT, 0, sb>>>(Sh);
     }
     if (core) {
       kernel_params(P, 0, S);

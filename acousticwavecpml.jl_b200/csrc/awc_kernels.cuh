@@ -308,6 +308,63 @@ struct Vec2<double> {
   using type = double2;
 };
 
+// Packed pairs of floats (f32x2): each half rounded like the scalar operation.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n .reg .b64 ra, rb, rc, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n"
+      " mov.b64 rc, {%6, %7};\n fma.rn.f32x2 rd, ra, rb, rc;\n mov.b64 {%0, %1}, rd;\n}\n"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n .reg .b64 ra, rb, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n"
+      " add.rn.f32x2 rd, ra, rb;\n mov.b64 {%0, %1}, rd;\n}\n"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n .reg .b64 ra, rb, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n"
+      " mul.rn.f32x2 rd, ra, rb;\n mov.b64 {%0, %1}, rd;\n}\n"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+// A product that a sum uses next: two scalar multiplies. ptxas contracts a
+// packed multiply into the packed add after it, with mul.rn and with
+// -fmad=false too, which changes the rounding.
+__device__ __forceinline__ float2 mul2_kept(float2 a, float b) {
+  return float2{mul_rn(a.x, b), mul_rn(a.y, b)};
+}
+// The two operations a second difference and a leapfrog take, on a pair of
+// nodes: m, c, p are the pair's neighbours along one axis and its values.
+__device__ __forceinline__ float2 pair_d2(float2 m, float2 c, float2 p, float inv_d2) {
+  return mul2_kept(add2(fma2(c, float2{-2.f, -2.f}, p), m), inv_d2);
+}
+__device__ __forceinline__ double2 pair_d2(double2 m, double2 c, double2 p, double inv_d2) {
+  return double2{second_diff(m.x, c.x, p.x, inv_d2), second_diff(m.y, c.y, p.y, inv_d2)};
+}
+__device__ __forceinline__ float2 pair_leapfrog3d(float2 c, float2 o, float2 f, float2 dx, float2 dy,
+                                                  float2 dz) {
+  const float2 lead{fmaf(2.f, c.x, -o.x), fmaf(2.f, c.y, -o.y)};
+  return fma2(f, add2(add2(dx, dy), dz), lead);
+}
+__device__ __forceinline__ double2 pair_leapfrog3d(double2 c, double2 o, double2 f, double2 dx,
+                                                   double2 dy, double2 dz) {
+  return double2{leapfrog3d(c.x, o.x, f.x, dx.x, dy.x, dz.x),
+                 leapfrog3d(c.y, o.y, f.y, dx.y, dy.y, dz.y)};
+}
+// Second differences along x of a pair with the values beside it.
+__device__ __forceinline__ float2 pair_d2x(float l, float2 c, float r, float inv_d2) {
+  return float2{mul_rn(fmaf(-2.f, c.x, c.y) + l, inv_d2), mul_rn(fmaf(-2.f, c.y, r) + c.x, inv_d2)};
+}
+__device__ __forceinline__ double2 pair_d2x(double l, double2 c, double r, double inv_d2) {
+  return double2{second_diff(l, c.x, c.y, inv_d2), second_diff(c.x, c.y, r, inv_d2)};
+}
+
 // Geometry of the 3D step kernel for element type T and TY thread rows:
 // a block of 32 x TY threads owns a 64 x 2TY tile of (x, y) nodes; thread
 // (tx, ty) owns the 2 x 2 nodes x0 + 2tx + {0,1}, y0 + 2ty + {0,1}. One
@@ -336,7 +393,8 @@ struct Tile3 {
 // warp is done with the stage). Plane k is computed from the stages of planes
 // k-1, k, k+1; loads run up to S-3 planes ahead and warps may drift apart by
 // as much, with no block-wide barrier in the loop. Each thread owns 2 x 2
-// nodes: an x pair read and written as one vector, in two rows.
+// nodes: an x pair read and written as one vector, in two rows, with its
+// values of planes k - 1 and k held in registers.
 template <typename T, int TY, int S>
 __global__ void __launch_bounds__(32 * TY) step3d_core(const __grid_constant__ CUtensorMap mc,
                                                        const __grid_constant__ CUtensorMap mo,
@@ -397,44 +455,46 @@ __global__ void __launch_bounds__(32 * TY) step3d_core(const __grid_constant__ C
   int64_t o = (int64_t)xa + px * j0 + plane * k0;  // pitched offset of node (xa, j0, k)
   int ioe = P.io.blk_off[blk];
   const int ioe1 = P.io.blk_off[blk + 1];
-  const int c0 = (2 * ty + 1) * L::PW + 2 * tx + L::A;  // pcur stage index of (xa, j0)
-  const int i0 = 2 * ty * L::TX + 2 * tx;               // pold/fact stage index of (xa, j0)
+  const int c0 = ((2 * ty + 1) * L::PW + 2 * tx + L::A) * (int)sizeof(T);  // (xa, j0) in a stage's pcur box
+  const int i0 = L::PC_PAD + (2 * ty * L::TX + 2 * tx) * (int)sizeof(T);   // and in its pold box
+  constexpr int RW = L::PW * (int)sizeof(T), RI = L::TX * (int)sizeof(T);  // row steps
   const T ix2 = P.inv_d2[0], iy2 = P.inv_d2[1], iz2 = P.inv_d2[2];
+  auto pair = [&](int at) { return *reinterpret_cast<const V2*>(smem + at); };
+  auto one = [&](int at) { return *reinterpret_cast<const T*>(smem + at); };
 
+  // Along z a thread keeps its own values of the planes k - 1 and k in
+  // registers: plane k reads only its own pair rows from plane k + 1's stage,
+  // and a stage is free once its plane has been computed.
   bool ok = mbar_wait(&full[0], 0, abort) && mbar_wait(&full[1 % S], (1 / S) & 1, abort);
-  int uc = 1;  // use index of the current plane
+  V2 zm0 = pair(c0), zm1 = pair(c0 + RW);
+  int sc = 1 % S;  // stage of plane k
+  int at = sc * L::BYTES;
+  V2 c_0 = pair(at + c0), c_1 = pair(at + c0 + RW);
+  __syncwarp();
+  if (tx == 0) mbar_arrive(&empty[0]);
+  int uc = 1;              // use index of the current plane
+  uint32_t par = (2 / S) & 1;  // parity of the next plane's use
   for (int k = k0; k < k1; ++k, ++uc, o += plane) {
-    ok = ok && mbar_wait(&full[(uc + 1) % S], ((uc + 1) / S) & 1, abort);
+    const int sn = sc + 1 == S ? 0 : sc + 1;
+    ok = ok && mbar_wait(&full[sn], par, abort);
     if (!ok) break;
-    const T* cm = reinterpret_cast<const T*>(smem + ((uc - 1) % S) * L::BYTES);
-    const T* cc = reinterpret_cast<const T*>(smem + (uc % S) * L::BYTES);
-    const T* cp = reinterpret_cast<const T*>(smem + ((uc + 1) % S) * L::BYTES);
-    const T* oo = reinterpret_cast<const T*>(smem + (uc % S) * L::BYTES + L::PC_PAD);
-    const T* ff = oo + L::TX * L::RY;
-    // rows j0 and j0+1: centre pairs, x apron scalars, y and z neighbours,
-    // pold and fact
-    const V2 c_0 = *reinterpret_cast<const V2*>(cc + c0);
-    const V2 c_1 = *reinterpret_cast<const V2*>(cc + c0 + L::PW);
-    const T xm0 = cc[c0 - 1], xp0 = cc[c0 + 2], xm1 = cc[c0 + L::PW - 1], xp1 = cc[c0 + L::PW + 2];
-    const V2 ym = *reinterpret_cast<const V2*>(cc + c0 - L::PW);
-    const V2 yp = *reinterpret_cast<const V2*>(cc + c0 + 2 * L::PW);
-    const V2 zm0 = *reinterpret_cast<const V2*>(cm + c0);
-    const V2 zm1 = *reinterpret_cast<const V2*>(cm + c0 + L::PW);
-    const V2 zp0 = *reinterpret_cast<const V2*>(cp + c0);
-    const V2 zp1 = *reinterpret_cast<const V2*>(cp + c0 + L::PW);
-    const V2 po0 = *reinterpret_cast<const V2*>(oo + i0);
-    const V2 po1 = *reinterpret_cast<const V2*>(oo + i0 + L::TX);
-    const V2 f_0 = *reinterpret_cast<const V2*>(ff + i0);
-    const V2 f_1 = *reinterpret_cast<const V2*>(ff + i0 + L::TX);
-    // node (row, x): 2 pcur - pold + fact * (d2x + d2y + d2z)
-    T v00 = leapfrog3d(c_0.x, po0.x, f_0.x, second_diff(xm0, c_0.x, c_0.y, ix2),
-                       second_diff(ym.x, c_0.x, c_1.x, iy2), second_diff(zm0.x, c_0.x, zp0.x, iz2));
-    T v01 = leapfrog3d(c_0.y, po0.y, f_0.y, second_diff(c_0.x, c_0.y, xp0, ix2),
-                       second_diff(ym.y, c_0.y, c_1.y, iy2), second_diff(zm0.y, c_0.y, zp0.y, iz2));
-    T v10 = leapfrog3d(c_1.x, po1.x, f_1.x, second_diff(xm1, c_1.x, c_1.y, ix2),
-                       second_diff(c_0.x, c_1.x, yp.x, iy2), second_diff(zm1.x, c_1.x, zp1.x, iz2));
-    T v11 = leapfrog3d(c_1.y, po1.y, f_1.y, second_diff(c_1.x, c_1.y, xp1, ix2),
-                       second_diff(c_0.y, c_1.y, yp.y, iy2), second_diff(zm1.y, c_1.y, zp1.y, iz2));
+    const int an = sn * L::BYTES;
+    // the next plane's rows j0 and j0+1; this plane's x aprons, rows above and
+    // below, pold and fact
+    const V2 zp0 = pair(an + c0), zp1 = pair(an + c0 + RW);
+    const T xm0 = one(at + c0 - (int)sizeof(T)), xp0 = one(at + c0 + 2 * (int)sizeof(T));
+    const T xm1 = one(at + c0 + RW - (int)sizeof(T)), xp1 = one(at + c0 + RW + 2 * (int)sizeof(T));
+    const V2 ym = pair(at + c0 - RW), yp = pair(at + c0 + 2 * RW);
+    const V2 po0 = pair(at + i0), po1 = pair(at + i0 + RI);
+    const V2 f_0 = pair(at + i0 + L::IN_BYTES), f_1 = pair(at + i0 + L::IN_BYTES + RI);
+    // this warp is done with the plane's stage; the producer may refill it
+    __syncwarp();
+    if (tx == 0) mbar_arrive(&empty[sc]);
+    // 2 pcur - pold + fact * (d2x + d2y + d2z)
+    V2 v0 = pair_leapfrog3d(c_0, po0, f_0, pair_d2x(xm0, c_0, xp0, ix2), pair_d2(ym, c_0, c_1, iy2),
+                            pair_d2(zm0, c_0, zp0, iz2));
+    V2 v1 = pair_leapfrog3d(c_1, po1, f_1, pair_d2x(xm1, c_1, xp1, ix2), pair_d2(c_0, c_1, yp, iy2),
+                            pair_d2(zm1, c_1, zp1, iz2));
     // sources and receivers of this plane (block-uniform walk, rarely taken)
     for (; ioe < ioe1; ++ioe) {
       const int4 en = P.io.ent[ioe];
@@ -442,24 +502,22 @@ __global__ void __launch_bounds__(32 * TY) step3d_core(const __grid_constant__ C
       const int lx = en.x & (L::TX - 1), ly = en.x / L::TX;
       if ((lx >> 1) == tx && (ly >> 1) == ty) {
         const int sub = ((ly & 1) << 1) | (lx & 1);
-        if (sub == 0) v00 = node_io(P.io, P.it, en.z, en.w, v00);
-        if (sub == 1) v01 = node_io(P.io, P.it, en.z, en.w, v01);
-        if (sub == 2) v10 = node_io(P.io, P.it, en.z, en.w, v10);
-        if (sub == 3) v11 = node_io(P.io, P.it, en.z, en.w, v11);
+        if (sub == 0) v0.x = node_io(P.io, P.it, en.z, en.w, v0.x);
+        if (sub == 1) v0.y = node_io(P.io, P.it, en.z, en.w, v0.y);
+        if (sub == 2) v1.x = node_io(P.io, P.it, en.z, en.w, v1.x);
+        if (sub == 3) v1.y = node_io(P.io, P.it, en.z, en.w, v1.y);
       }
     }
-    // this warp is done with stage uc-1; the producer may refill it
-    __syncwarp();
-    if (tx == 0) mbar_arrive(&empty[(uc - 1) % S]);
     if (all4) {
-      *reinterpret_cast<V2*>(P.pnew + o) = V2{v00, v01};
-      *reinterpret_cast<V2*>(P.pnew + o + px) = V2{v10, v11};
+      *reinterpret_cast<V2*>(P.pnew + o) = v0;
+      *reinterpret_cast<V2*>(P.pnew + o + px) = v1;
     } else if (any) {
-      if (vx0) P.pnew[o] = v00;
-      if (vx1) P.pnew[o + 1] = v01;
-      if (vy1 && vx0) P.pnew[o + px] = v10;
-      if (vy1 && vx1) P.pnew[o + px + 1] = v11;
+      if (vx0) P.pnew[o] = v0.x;
+      if (vx1) P.pnew[o + 1] = v0.y;
+      if (vy1 && vx0) P.pnew[o + px] = v1.x;
+      if (vy1 && vx1) P.pnew[o + px + 1] = v1.y;
     }
+    // refill the stage the whole block left in the last iteration
     if (tid == 0 && uc - 1 + S < nplanes) {
       if (!mbar_wait(&empty[(uc - 1) % S], ((uc - 1) / S) & 1, abort)) {
         ok = false;
@@ -467,6 +525,13 @@ __global__ void __launch_bounds__(32 * TY) step3d_core(const __grid_constant__ C
       }
       issue(uc - 1 + S);
     }
+    zm0 = c_0;
+    zm1 = c_1;
+    c_0 = zp0;
+    c_1 = zp1;
+    sc = sn;
+    at = an;
+    if (sn == S - 1) par ^= 1;
   }
   if (!ok) {
     // a wait ran out: record it, stop the block, and let the producer drain
@@ -505,6 +570,15 @@ __device__ __forceinline__ void band_apply(const BandSide<T>& B, const BandCoef<
 // columns and streams a chunk of P.shell_zchunk planes of them, keeping each
 // column's z neighbours in registers.
 //
+// What bounds it is the latency of the loads of a plane (305 MB of DRAM
+// traffic per step at 296 x 276 x 296 in FP32, 76 us alone). So on grids with
+// enough columns for it (see band_wide in awc_api.cu) PAIR gives the threads of
+// the y and z slabs two nodes each, and every thread asks L2 for the next
+// plane's single-use data while it computes this one. With the core kernel
+// beside it a step took 135.8 us before, 135.3 with pairs alone, 126.7 with
+// both (FP64, 203 x 187 x 171: 97.7, 89.6, 84.8 us); asking two or three
+// planes ahead 125.5 and 126.6 us, but 87.7 and 89.4 us in FP64.
+//
 // Box.kind says which bands the nodes of a box lie in, and the block body is
 // compiled per kind:
 //   1  an x slab: every node lies in the x band of the slab's side;
@@ -527,10 +601,12 @@ __device__ __forceinline__ void band_apply(const BandSide<T>& B, const BandCoef<
 constexpr int BAND_NT = 128;
 
 // Blocks of BAND_NT threads per SM the band kernel is compiled for (its
-// register budget: 65536 / (BAND_NT * blocks) per thread).
-template <typename T>
+// register budget: 65536 / (BAND_NT * blocks) per thread). Pairs in FP32 at 296
+// x 276 x 296 with 6, 7 and 8 blocks: 128.8, 126.7 and 130.3 us per step; in
+// FP64 4 blocks (5: no faster).
+template <typename T, bool PAIR>
 struct BandOcc {
-  static constexpr int blocks = (sizeof(T) == 4 ? 1024 : 512) / BAND_NT;
+  static constexpr int blocks = sizeof(T) == 4 ? (PAIR ? 7 : 8) : 4;
 };
 
 // Coefficients of entry q from the left side's arrays L: hq = half-grid index
@@ -554,7 +630,12 @@ struct ColBand {
   I pq = 0, xq = 0;
 };
 
-template <typename T, typename I, int KIND>
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
+// One node per thread. AHEAD: x slabs ask L2 for the next plane's data.
+template <typename T, typename I, int KIND, bool AHEAD>
 __device__ __forceinline__ void band_body(const StepParams<T>& P, int blk, const Box& B, int r) {
   constexpr bool GEN = KIND == 15;
   constexpr bool XPRIM = KIND == 1, YPRIM = KIND == 3;  // the slab's own axis
@@ -625,6 +706,13 @@ __device__ __forceinline__ void band_body(const StepParams<T>& P, int blk, const
     if (valid) {
       pp = __ldg(pcur + (o + plane));
       const T po = __ldg(P.pold + o), f = __ldg(P.fact + o);
+      if (AHEAD && XPRIM && k + 1 < k1) {
+        prefetch_l2(pcur + (o + 2 * plane));
+        prefetch_l2(P.pold + (o + plane));
+        prefetch_l2(P.fact + (o + plane));
+        prefetch_l2(LX.psi_old + (X.pq + (I)P.psi_dz[0]));
+        prefetch_l2(LX.xi + (X.xq + (I)P.xi_dz[0]));
+      }
       // offsets of this plane's x and y entries
       I xpq = X.pq, xxq = X.xq, ypq = Y.pq, yxq = Y.xq;
       if ((KIND & 1) && !XPRIM && X.s) {
@@ -713,8 +801,183 @@ __device__ __forceinline__ void band_body(const StepParams<T>& P, int blk, const
   }
 }
 
-template <typename T, typename I>
-__global__ void __launch_bounds__(BAND_NT, BandOcc<T>::blocks) step3d_band(StepParams<T> P) {
+// y slabs (kind 3) and z slabs (kind 7), two nodes of a row per thread: the
+// pair (i, i + 1), i even, is one aligned vector in every field and in the ψ
+// and ξ arrays of y and z, whose rows have the fields' pitch. Half the loads
+// and addresses of one node per thread, twice the bytes in flight per warp.
+// Columns outside the box (the Dirichlet ones beside a pair's interior node)
+// are computed and not stored, except their ψ and ξ, which nothing reads.
+template <typename T, typename I, int KIND>
+__device__ __forceinline__ void band_pair(const StepParams<T>& P, int blk, const Box& B, int r) {
+  using V2 = typename Vec2<T>::type;
+  constexpr bool YPRIM = KIND == 3;
+  const int xs0 = B.x0 & ~1;
+  const int W = ((B.x1 - xs0) >> 1) + 1;
+  const int ncol = W * (B.y1 - B.y0 + 1);
+  const int ncb = (ncol + BAND_NT - 1) / BAND_NT;
+  const int l = (r % ncb) * BAND_NT + (int)threadIdx.x;
+  const int k0 = B.z0 + (r / ncb) * P.shell_zchunk;
+  const int k1 = min(k0 + P.shell_zchunk, B.z1 + 1);
+  const bool valid = l < ncol;
+  const int i = xs0 + 2 * (valid ? l % W : 0), j = B.y0 + (valid ? l / W : 0);
+  const bool v0 = valid && i >= B.x0, v1 = valid && i + 1 <= B.x1;
+  const int halo = P.halo;
+  const I px = (I)P.px, plane = (I)P.plane;
+  I o = (I)i + px * (I)j + plane * (I)k0;
+  int ioe = P.io.blk_off[blk];
+  const int ioe1 = P.io.blk_off[blk + 1];
+  const BandSide<T>&LX = P.band[0][0], &LY = P.band[1][0], &LZ = P.band[2][0];
+  // whether a node of the pair lies in an active x band, the y band's entry
+  const bool xb = valid && ((P.active[0][0] && i <= halo) ||
+                            (P.active[0][1] && i + 1 >= P.nx - halo - 1));
+  int yq_ = 0, ys = 0;
+  bool yfirst = false;
+  if (valid) {
+    ys = band_of(j, P.ny, halo, P.first_r[1], yq_, yfirst);
+    if (!YPRIM && ys != 0 && !(ys == 1 ? P.active[1][0] : P.active[1][1])) ys = 0;
+  }
+  const bool yR = ys == 2;
+  // ψ[q] and ξ[q-1] of the y band at the plane k0, and their step to the next
+  I ypq = (I)i + px * ((I)yq_ + (I)(halo + 1) * (I)k0) + (yR ? (I)P.psi_side[1] : (I)0);
+  I yxq = (I)i + px * ((I)(yq_ - 1) + (I)halo * (I)k0) + (yR ? (I)P.xi_side[1] : (I)0);
+  const I dyp = (I)P.psi_dz[1], dyx = (I)P.xi_dz[1];
+  // z slab: ψ[q] of node (i, j, k) at o - zsp and ξ[q-1] at o - plane - zsx
+  I zsp = 0, zsx = 0;
+  if (KIND == 7 && B.z0 != 1) {
+    const I zs = plane * (I)(P.nz - halo - 2);
+    zsp = zs - (I)P.psi_side[2];
+    zsx = zs - (I)P.xi_side[2];
+  }
+  const T* __restrict__ pcur = P.pcur;
+  auto ld2 = [](const T* q) { return __ldg(reinterpret_cast<const V2*>(q)); };
+  auto rd2 = [](const T* q) { return *reinterpret_cast<const V2*>(q); };
+  auto st2 = [](T* q, T a, T b) { *reinterpret_cast<V2*>(q) = V2{a, b}; };
+  V2 pm{}, pc{}, zc{};  // zc: new ψ on the upper z face of the previous plane's nodes
+  if (valid) {
+    pm = ld2(pcur + (o - plane));
+    pc = ld2(pcur + o);
+  }
+  for (int k = k0; k < k1; ++k, o += plane, ypq += dyp, yxq += dyx) {
+    int sz = 0, qz = 0;
+    bool fz = false;
+    if (KIND == 7) sz = band_of(k, P.nz, halo, P.first_r[2], qz, fz);
+    const bool zR = sz == 2, zcarry = k > k0 && !fz;
+    V2 pp{};
+    T a = 0, b = 0;
+    if (valid) {
+      pp = ld2(pcur + (o + plane));
+      const V2 po = ld2(P.pold + o), f = ld2(P.fact + o);
+      if (k + 1 < k1) {  // the next plane's single-use data
+        prefetch_l2(pcur + (o + 2 * plane));
+        prefetch_l2(P.pold + (o + plane));
+        prefetch_l2(P.fact + (o + plane));
+        if (KIND == 7) {
+          prefetch_l2(LZ.psi_old + (o - zsp + plane));
+          prefetch_l2(LZ.xi + (o - zsx));
+        }
+        if (YPRIM) {
+          prefetch_l2(LY.psi_old + (ypq + dyp));
+          prefetch_l2(LY.xi + (yxq + dyx));
+        }
+      }
+      const V2 ym = ld2(pcur + (o - px)), yp = ld2(pcur + (o + px));
+      const T xm = __ldg(pcur + (o - 1)), xp = __ldg(pcur + (o + 2));
+      const I zp = o - zsp, zxo = o - plane - zsx;
+      V2 zq{}, zm{}, zx{}, yq{}, ymq{}, yx{};
+      if (KIND == 7) {
+        zq = rd2(LZ.psi_old + zp);
+        zx = rd2(LZ.xi + zxo);
+        if (!zcarry) zm = rd2(LZ.psi_old + (zp - plane));
+      }
+      if (YPRIM || ys) {
+        yq = rd2(LY.psi_old + ypq);
+        ymq = rd2(LY.psi_old + (ypq - px));
+        yx = rd2(LY.xi + yxq);
+      }
+      const T dxa = second_diff(xm, pc.x, pc.y, P.inv_d2[0]);
+      const T dxb = second_diff(pc.x, pc.y, xp, P.inv_d2[0]);
+      const T dya = second_diff(ym.x, pc.x, yp.x, P.inv_d2[1]);
+      const T dyb = second_diff(ym.y, pc.y, yp.y, P.inv_d2[1]);
+      const T dza = second_diff(pm.x, pc.x, pp.x, P.inv_d2[2]);
+      const T dzb = second_diff(pm.y, pc.y, pp.y, P.inv_d2[2]);
+      a = leapfrog3d(pc.x, po.x, f.x, dxa, dya, dza);
+      b = leapfrog3d(pc.y, po.y, f.y, dxb, dyb, dzb);
+      T da = 0, db = 0;
+      if (xb) {  // x terms, node by node
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          int q;
+          bool first;
+          const int c = i + n;
+          const int s = band_of(c, P.nx, halo, P.first_r[0], q, first);
+          if (!(n ? v1 : v0) || s == 0 || !(s == 1 ? P.active[0][0] : P.active[0][1])) continue;
+          const bool R = s == 2;
+          const I jk = (I)j + (I)P.ny * (I)k;
+          const I pq = (I)(halo + 1) * jk + (I)q + (R ? (I)P.psi_side[0] : (I)0);
+          const I xq = (I)halo * jk + (I)(q - 1) + (R ? (I)P.xi_side[0] : (I)0);
+          band_apply(LX, coef_at(LX, q + (R ? halo + 1 : 0), q - 1 + (R ? halo : 0)), first, pq,
+                     (I)1, xq, LX.psi_old[pq], LX.psi_old[pq - 1], LX.xi[xq], n ? pc.x : xm,
+                     n ? pc.y : pc.x, n ? xp : pc.y, n ? dxb : dxa, n ? f.y : f.x, P.inv_d[0],
+                     n ? db : da);
+        }
+      }
+      if (YPRIM || ys) {
+        const T inv = P.inv_d[1];
+        const BandCoef<T> c = coef_at(LY, yq_ + (yR ? halo + 1 : 0), yq_ - 1 + (yR ? halo : 0));
+        T qa, qb, ma, mb, xa, xb2;
+        cpml_axis(c, yq.x, ymq.x, yx.x, ym.x, pc.x, yp.x, dya, f.x, inv, qa, ma, xa, da);
+        cpml_axis(c, yq.y, ymq.y, yx.y, ym.y, pc.y, yp.y, dyb, f.y, inv, qb, mb, xb2, db);
+        st2(LY.psi_new + ypq, qa, qb);
+        if (yfirst) st2(LY.psi_new + (ypq - px), ma, mb);
+        st2(LY.xi + yxq, xa, xb2);
+      }
+      if (KIND == 7) {
+        const T inv = P.inv_d[2];
+        const int hq = qz + (zR ? halo + 1 : 0), g = qz - 1 + (zR ? halo : 0);
+        const T bh = __ldg(LZ.bKh + hq), ah = __ldg(LZ.ah + hq);
+        const T bk = __ldg(LZ.bK + g), ak = __ldg(LZ.a + g);
+        if (!zcarry) {
+          const T bm = __ldg(LZ.bKh + hq - 1), am = __ldg(LZ.ah + hq - 1);
+          zc.x = psi_face(bm, am, zm.x, pc.x - pm.x, inv);
+          zc.y = psi_face(bm, am, zm.y, pc.y - pm.y, inv);
+        }
+        const T qa = psi_face(bh, ah, zq.x, pp.x - pc.x, inv);
+        const T qb = psi_face(bh, ah, zq.y, pp.y - pc.y, inv);
+        T xa, xb2;
+        cpml_tail(bk, ak, qa, zc.x, zx.x, dza, f.x, inv, xa, da);
+        cpml_tail(bk, ak, qb, zc.y, zx.y, dzb, f.y, inv, xb2, db);
+        st2(LZ.psi_new + zp, qa, qb);
+        if (fz) st2(LZ.psi_new + (zp - plane), zc.x, zc.y);
+        st2(LZ.xi + zxo, xa, xb2);
+        zc = V2{qa, qb};
+      }
+      a += da;
+      b += db;
+    }
+    // sources and receivers of this plane (block-uniform walk)
+    for (; ioe < ioe1; ++ioe) {
+      const int4 en = P.io.ent[ioe];
+      if (en.y != k) break;
+      if (valid && (en.x >> 1) == (int)threadIdx.x) {
+        if (en.x & 1)
+          b = node_io(P.io, P.it, en.z, en.w, b);
+        else
+          a = node_io(P.io, P.it, en.z, en.w, a);
+      }
+    }
+    if (v0 && v1) {
+      st2(P.pnew + o, a, b);
+    } else {
+      if (v0) P.pnew[o] = a;
+      if (v1) P.pnew[o + 1] = b;
+    }
+    pm = pc;
+    pc = pp;
+  }
+}
+
+template <typename T, typename I, bool PAIR>
+__global__ void __launch_bounds__(BAND_NT, BandOcc<T, PAIR>::blocks) step3d_band(StepParams<T> P) {
   const int blk = (int)blockIdx.x;
   if (blk == 0 && P.do_rim && P.io.nrim > 0) rim_io(P.io, P.pnew, P.it);
   int b = 0;
@@ -722,13 +985,17 @@ __global__ void __launch_bounds__(BAND_NT, BandOcc<T>::blocks) step3d_band(StepP
   const Box B = P.box[b];
   const int r = blk - P.box_blk[b];
   if (B.kind == 1)
-    band_body<T, I, 1>(P, blk, B, r);
+    band_body<T, I, 1, PAIR>(P, blk, B, r);
+  else if (B.kind == 3 && PAIR)
+    band_pair<T, I, 3>(P, blk, B, r);
   else if (B.kind == 3)
-    band_body<T, I, 3>(P, blk, B, r);
+    band_body<T, I, 3, false>(P, blk, B, r);
+  else if (B.kind == 7 && PAIR)
+    band_pair<T, I, 7>(P, blk, B, r);
   else if (B.kind == 7)
-    band_body<T, I, 7>(P, blk, B, r);
+    band_body<T, I, 7, false>(P, blk, B, r);
   else
-    band_body<T, I, 15>(P, blk, B, r);
+    band_body<T, I, 15, false>(P, blk, B, r);
 }
 
 // ---------------------------------------------------------------------------

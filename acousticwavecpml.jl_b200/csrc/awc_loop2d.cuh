@@ -280,36 +280,6 @@ __device__ __forceinline__ bool mail_take(const unsigned long long* q, uint32_t 
 // nodes per instruction (packed f32x2, each half rounded like the scalar
 // operation): 28 instead of 36 instructions per 4 nodes. The x neighbours of
 // a pair straddle register pairs, so the x part stays scalar.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("{\n .reg .b64 ra, rb, rc, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n"
-      " mov.b64 rc, {%6, %7};\n fma.rn.f32x2 rd, ra, rb, rc;\n mov.b64 {%0, %1}, rd;\n}\n"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return d;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n .reg .b64 ra, rb, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n"
-      " add.rn.f32x2 rd, ra, rb;\n mov.b64 {%0, %1}, rd;\n}\n"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n .reg .b64 ra, rb, rd;\n mov.b64 ra, {%2, %3};\n mov.b64 rb, {%4, %5};\n"
-      " mul.rn.f32x2 rd, ra, rb;\n mov.b64 {%0, %1}, rd;\n}\n"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-// A product that a sum uses next: two scalar multiplies. ptxas contracts a
-// packed multiply into the packed add after it, with mul.rn and with
-// -fmad=false too, which changes the rounding.
-__device__ __forceinline__ float2 mul2_kept(float2 a, float b) {
-  return float2{mul_rn(a.x, b), mul_rn(a.y, b)};
-}
 __device__ __forceinline__ void vec_update(const Pack<float>& up, const Pack<float>& c,
                                            const Pack<float>& dn, const Pack<float>& o,
                                            const Pack<float>& f, float xm, float xp, float ix2,
