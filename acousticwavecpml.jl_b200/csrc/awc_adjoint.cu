@@ -47,7 +47,9 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <map>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "../../include/awcpml.h"
@@ -191,9 +193,9 @@ __device__ __forceinline__ T adj_g(const AdjStep<T>& A, I o) {
 // precision) at nodes outside every active band, (p_{t+1} - 2 p_t + p_{t-1})
 // / F (in double) inside one, where adj_sources removes the source term.
 template <typename T, typename I, int ND, bool GRAD>
-__device__ __forceinline__ void adj_update(const AdjStep<T>& A, I o, T l2, T f, T lap, T band,
-                                           bool in_band) {
-  const T lam = (T(2) * l2 - A.lam[o]) + (lap + band);
+__device__ __forceinline__ T adj_update(const AdjStep<T>& A, I o, T l2, T l3, T f, T lap, T band,
+                                        bool in_band) {
+  const T lam = (T(2) * l2 - l3) + (lap + band);
   if (GRAD) {
     const T* __restrict__ P = A.p0;
     const T c = __ldg(P + o);
@@ -219,14 +221,15 @@ __device__ __forceinline__ void adj_update(const AdjStep<T>& A, I o, T l2, T f, 
     A.grad[o] += (double)lam * b;
   }
   A.lam[o] = lam;
+  return lam;
 }
 
-// Nodes of the core box: blocks of 32 x 8 (x, y) nodes of one z plane.
-template <typename T, typename I, int ND, bool GRAD>
+// Nodes of the 3D core box: blocks of 32 x 8 (x, y) nodes of one z plane.
+template <typename T, typename I, bool GRAD>
 __global__ void __launch_bounds__(256) adj_core(const __grid_constant__ AdjStep<T> A) {
   const int i = A.core.x0 + blockIdx.x * 32 + threadIdx.x;
   const int j = A.core.y0 + blockIdx.y * 8 + threadIdx.y;
-  const int k = ND == 3 ? A.core.z0 + (int)blockIdx.z : 0;
+  const int k = A.core.z0 + (int)blockIdx.z;
   if (i > A.core.x1 || j > A.core.y1) return;
   const I px = (I)A.px, pl = (I)A.plane;
   const I o = (I)i + px * (I)j + pl * (I)k;
@@ -234,16 +237,15 @@ __global__ void __launch_bounds__(256) adj_core(const __grid_constant__ AdjStep<
   const T gc = mul_rn(f, l2);
   T lap = second_diff(adj_g(A, o - 1), gc, adj_g(A, o + 1), A.inv_d2[0]) +
           second_diff(adj_g(A, o - px), gc, adj_g(A, o + px), A.inv_d2[1]);
-  if (ND == 3) lap += second_diff(adj_g(A, o - pl), gc, adj_g(A, o + pl), A.inv_d2[2]);
-  adj_update<T, I, ND, GRAD>(A, o, l2, f, lap, T(0), false);
+  lap += second_diff(adj_g(A, o - pl), gc, adj_g(A, o + pl), A.inv_d2[2]);
+  adj_update<T, I, 3, GRAD>(A, o, l2, A.lam[o], f, lap, T(0), false);
 }
 
 // One shell node whose band zone per axis is ZX, ZY, ZZ (0 none, 1 left, 2
 // right; 3 unknown: both sides tested at run time).
 template <typename T, typename I, int ND, bool GRAD, int ZX, int ZY, int ZZ>
-__device__ __forceinline__ void adj_shell_node(const AdjStep<T>& A, int i, int j, int k) {
+__device__ __forceinline__ T adj_shell_node(const AdjStep<T>& A, int i, int j, int k, I o, T l3) {
   const I px = (I)A.px, pl = (I)A.plane;
-  const I o = (I)i + px * (I)j + pl * (I)k;
   const T f = __ldg(A.F + o), l2 = __ldg(A.lam2 + o);
   const T gc = mul_rn(f, l2);
   const T g[3][2] = {{adj_g(A, o - 1), adj_g(A, o + 1)},
@@ -267,13 +269,13 @@ __device__ __forceinline__ void adj_shell_node(const AdjStep<T>& A, int i, int j
       band += adj_side<T, I>(A, a, s, q, i, j, k, g[a][0], gc, g[a][1]);
     }
   }
-  adj_update<T, I, ND, GRAD>(A, o, l2, f, lap, band, in_band);
+  return adj_update<T, I, ND, GRAD>(A, o, l2, l3, f, lap, band, in_band);
 }
 
 // Nodes of the shell boxes: a box's (x, y) columns numbered row by row,
 // l = (i - x0) + W (j - y0), in runs of 256 per block, one z plane per block;
 // the block's box kind selects the body.
-template <typename T, typename I, int ND, bool GRAD>
+template <typename T, typename I, bool GRAD>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4) adj_shell(const __grid_constant__ AdjStep<T> A) {
   // the box of this block: box_blk rises strictly, so a binary search
   const int blk = blockIdx.x;
@@ -293,28 +295,84 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4) adj_shell(const _
   const int l = (r - kz * ncb) * 256 + threadIdx.x;
   if (l >= ncol) return;
   const int jl = A.fastdiv ? (int)(((uint64_t)l * A.box_mw[b]) >> 32) : l / W;
-  const int i = B.x0 + (l - jl * W), j = B.y0 + jl, k = ND == 3 ? B.z0 + kz : 0;
+  const int i = B.x0 + (l - jl * W), j = B.y0 + jl, k = B.z0 + kz;
+  const I o = (I)i + (I)A.px * (I)j + (I)A.plane * (I)k;
 #define AWC_SHELL(zx, zy, zz) \
-  case (zx) + 3 * (zy) + 9 * (zz): adj_shell_node<T, I, ND, GRAD, zx, zy, zz>(A, i, j, k); break;
-  if (ND == 2) {
-    switch (B.kind) {
-      AWC_SHELL(1, 0, 0) AWC_SHELL(2, 0, 0) AWC_SHELL(0, 1, 0) AWC_SHELL(1, 1, 0)
-      AWC_SHELL(2, 1, 0) AWC_SHELL(0, 2, 0) AWC_SHELL(1, 2, 0) AWC_SHELL(2, 2, 0)
-      default: adj_shell_node<T, I, ND, GRAD, 3, 3, 0>(A, i, j, k);
-    }
-  } else {
-    switch (B.kind) {
-      AWC_SHELL(1, 0, 0) AWC_SHELL(2, 0, 0) AWC_SHELL(0, 1, 0) AWC_SHELL(1, 1, 0)
-      AWC_SHELL(2, 1, 0) AWC_SHELL(0, 2, 0) AWC_SHELL(1, 2, 0) AWC_SHELL(2, 2, 0)
-      AWC_SHELL(0, 0, 1) AWC_SHELL(1, 0, 1) AWC_SHELL(2, 0, 1) AWC_SHELL(0, 1, 1)
-      AWC_SHELL(1, 1, 1) AWC_SHELL(2, 1, 1) AWC_SHELL(0, 2, 1) AWC_SHELL(1, 2, 1)
-      AWC_SHELL(2, 2, 1) AWC_SHELL(0, 0, 2) AWC_SHELL(1, 0, 2) AWC_SHELL(2, 0, 2)
-      AWC_SHELL(0, 1, 2) AWC_SHELL(1, 1, 2) AWC_SHELL(2, 1, 2) AWC_SHELL(0, 2, 2)
-      AWC_SHELL(1, 2, 2) AWC_SHELL(2, 2, 2)
-      default: adj_shell_node<T, I, ND, GRAD, 3, 3, 3>(A, i, j, k);
-    }
+  case (zx) + 3 * (zy) + 9 * (zz): \
+    adj_shell_node<T, I, 3, GRAD, zx, zy, zz>(A, i, j, k, o, A.lam[o]); \
+    break;
+  switch (B.kind) {
+    AWC_SHELL(1, 0, 0) AWC_SHELL(2, 0, 0) AWC_SHELL(0, 1, 0) AWC_SHELL(1, 1, 0)
+    AWC_SHELL(2, 1, 0) AWC_SHELL(0, 2, 0) AWC_SHELL(1, 2, 0) AWC_SHELL(2, 2, 0)
+    AWC_SHELL(0, 0, 1) AWC_SHELL(1, 0, 1) AWC_SHELL(2, 0, 1) AWC_SHELL(0, 1, 1)
+    AWC_SHELL(1, 1, 1) AWC_SHELL(2, 1, 1) AWC_SHELL(0, 2, 1) AWC_SHELL(1, 2, 1)
+    AWC_SHELL(2, 2, 1) AWC_SHELL(0, 0, 2) AWC_SHELL(1, 0, 2) AWC_SHELL(2, 0, 2)
+    AWC_SHELL(0, 1, 2) AWC_SHELL(1, 1, 2) AWC_SHELL(2, 1, 2) AWC_SHELL(0, 2, 2)
+    AWC_SHELL(1, 2, 2) AWC_SHELL(2, 2, 2)
+    default: adj_shell_node<T, I, 3, GRAD, 3, 3, 3>(A, i, j, k, o, A.lam[o]);
   }
 #undef AWC_SHELL
+}
+
+// The receiver and source nodes of a 2D step: `flag` marks them (one byte per
+// pitched node), `node` lists them in increasing order, and node n has the
+// receivers rids[roff[n] .. roff[n+1]) and sources sids[soff[n] .. soff[n+1]),
+// each in increasing order. res, stf and out are the step's rows.
+template <typename T>
+struct AdjIo2 {
+  const uint8_t* flag;
+  const int64_t* node;
+  const int32_t *roff, *rids, *soff, *sids;
+  int32_t n;
+  const int8_t* in_band;  // per source
+  const T *res, *stf;
+  T* out;
+};
+
+// A whole 2D adjoint step in one launch: one thread per interior node, with
+// its receivers' residuals entering λ_{t+3} first and its sources served from
+// its new value (adj_residuals and adj_sources, node by node). A 2D step is a
+// few hundred thousand nodes, so what it costs is launches: as four of them on
+// two streams it took 17 us, bound by the host, against 2.4 us in this form
+// (540 x 296, FP32). The launches overlap: the next step's blocks come up while
+// this one drains (programmatic dependent launch) and wait for its end here.
+template <typename T, typename I, bool GRAD>
+__global__ void __launch_bounds__(256) adj_step2d(const __grid_constant__ AdjStep<T> A,
+                                                  const __grid_constant__ AdjIo2<T> Q) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int i = 1 + (int)(blockIdx.x * 32 + threadIdx.x), j = 1 + (int)(blockIdx.y * 8 + threadIdx.y);
+  if (i > A.nx - 2 || j > A.ny - 2) return;
+  const I o = (I)i + (I)A.px * (I)j;
+  T l3 = A.lam[o];
+  int g = -1;
+  if (__ldg(Q.flag + o)) {
+    int lo = 0, hi = Q.n - 1;  // the node is in the list
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (Q.node[mid] < (int64_t)o)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    g = lo;
+    for (int e = Q.roff[g]; e < Q.roff[g + 1]; ++e) l3 -= Q.res[Q.rids[e]];
+  }
+  const T lam = adj_shell_node<T, I, 2, GRAD, 3, 3, 0>(A, i, j, 0, o, l3);
+  if (g >= 0)
+    for (int e = Q.soff[g]; e < Q.soff[g + 1]; ++e) {
+      const int s = Q.sids[e];
+      if (Q.out) Q.out[s] = lam;
+      // only band nodes use the difference form of the bracket, which holds S_t
+      if (GRAD && Q.in_band[s])
+        A.grad[o] -= (double)lam * (double)Q.stf[s] / (double)A.F[o];
+    }
+}
+
+// Marks the listed nodes in a zeroed flag array.
+__global__ void adj_mark(uint8_t* flag, const int64_t* node, int32_t n) {
+  const int k = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (k < n) flag[node[k]] = 1;
 }
 
 // Geometry of the TMA-fed core kernel (32 x TY threads, a 64 x 2TY tile of
@@ -826,47 +884,41 @@ void adj_regions(awc::AdjStep<T>& A, int ndim) {
 }
 
 // Offsets fit in int32 when every field (and so every band array) does.
-template <typename T, int ND, bool GRAD>
-void launch_core_i(const awc::AdjStep<T>& A, bool i64, dim3 grid, cudaStream_t st) {
-  if (i64)
-    awc::adj_core<T, int64_t, ND, GRAD><<<grid, dim3(32, 8), 0, st>>>(A);
-  else
-    awc::adj_core<T, int32_t, ND, GRAD><<<grid, dim3(32, 8), 0, st>>>(A);
+template <typename T>
+void launch_core(const awc::AdjStep<T>& A, bool grad, bool i64, dim3 grid, cudaStream_t st) {
+  const auto k = grad ? (i64 ? awc::adj_core<T, int64_t, true> : awc::adj_core<T, int32_t, true>)
+                      : (i64 ? awc::adj_core<T, int64_t, false> : awc::adj_core<T, int32_t, false>);
+  k<<<grid, dim3(32, 8), 0, st>>>(A);
 }
 
 template <typename T>
-void launch_core(const awc::AdjStep<T>& A, int ndim, bool grad, bool i64, dim3 grid,
-                 cudaStream_t st) {
-  if (ndim == 3 && grad)
-    launch_core_i<T, 3, true>(A, i64, grid, st);
-  else if (ndim == 3)
-    launch_core_i<T, 3, false>(A, i64, grid, st);
-  else if (grad)
-    launch_core_i<T, 2, true>(A, i64, grid, st);
-  else
-    launch_core_i<T, 2, false>(A, i64, grid, st);
+void launch_shell(const awc::AdjStep<T>& A, bool grad, bool i64, unsigned blocks, cudaStream_t st) {
+  const auto k = grad ? (i64 ? awc::adj_shell<T, int64_t, true> : awc::adj_shell<T, int32_t, true>)
+                      : (i64 ? awc::adj_shell<T, int64_t, false> : awc::adj_shell<T, int32_t, false>);
+  k<<<blocks, 256, 0, st>>>(A);
 }
 
-template <typename T, int ND, bool GRAD>
-void launch_shell_i(const awc::AdjStep<T>& A, bool i64, unsigned blocks, cudaStream_t st) {
-  if (i64)
-    awc::adj_shell<T, int64_t, ND, GRAD><<<blocks, 256, 0, st>>>(A);
-  else
-    awc::adj_shell<T, int32_t, ND, GRAD><<<blocks, 256, 0, st>>>(A);
-}
-
+// One 2D step, as a programmatic dependent of the kernel before it.
 template <typename T>
-void launch_shell(const awc::AdjStep<T>& A, int ndim, bool grad, bool i64, unsigned blocks,
-                  cudaStream_t st) {
-  if (ndim == 3 && grad)
-    launch_shell_i<T, 3, true>(A, i64, blocks, st);
-  else if (ndim == 3)
-    launch_shell_i<T, 3, false>(A, i64, blocks, st);
-  else if (grad)
-    launch_shell_i<T, 2, true>(A, i64, blocks, st);
-  else
-    launch_shell_i<T, 2, false>(A, i64, blocks, st);
+cudaError_t launch_2d(const awc::AdjStep<T>& A, const awc::AdjIo2<T>& Q, bool grad, bool i64,
+                      cudaStream_t st) {
+  const auto k = grad ? (i64 ? awc::adj_step2d<T, int64_t, true> : awc::adj_step2d<T, int32_t, true>)
+                      : (i64 ? awc::adj_step2d<T, int64_t, false> : awc::adj_step2d<T, int32_t, false>);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)((A.nx - 2 + 31) / 32), (unsigned)((A.ny - 2 + 7) / 8));
+  cfg.blockDim = dim3(32, 8);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, A, Q);
 }
+
+// Fields of a whole run kept instead of recomputed by segments up to this size
+// (540 x 296, FP32, 600 steps: 0.4 GB).
+constexpr int64_t KEEP_ALL = (int64_t)1 << 30;
 
 // TMA-fed core kernel: tile 64 x 8 nodes, 4 stages.
 constexpr int ADJ_TY = 4, ADJ_STAGES = 4;
@@ -992,6 +1044,55 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
   int8_t* sband_d;
   ADJ_TRY(C, mem.get(&sband_d, sband.size()));
   ADJ_TRY(C, cudaMemcpyAsync(sband_d, sband.data(), sband.size(), cudaMemcpyHostToDevice, st));
+  // 2D: the receiver and source nodes by node (see AdjIo2)
+  awc::AdjIo2<T> IO{};
+  std::vector<int64_t> io_node;
+  std::vector<int32_t> io_roff{0}, io_rids, io_soff{0}, io_sids;
+  if (p->ndim == 2) {
+    std::map<int64_t, std::pair<std::vector<int32_t>, std::vector<int32_t>>> by;
+    for (size_t g = 0; g < RG.node.size(); ++g)
+      by[RG.node[g]].first.assign(RG.ids.begin() + RG.off[g], RG.ids.begin() + RG.off[g + 1]);
+    for (int64_t s = 0; s < nsrc; ++s)
+      if (snode[s] >= 0) by[snode[s]].second.push_back((int32_t)s);
+    for (const auto& e : by) {
+      io_node.push_back(e.first);
+      io_rids.insert(io_rids.end(), e.second.first.begin(), e.second.first.end());
+      io_sids.insert(io_sids.end(), e.second.second.begin(), e.second.second.end());
+      io_roff.push_back((int32_t)io_rids.size());
+      io_soff.push_back((int32_t)io_sids.size());
+    }
+    // one block: node list, the four lists, the flags
+    const size_t n = io_node.size(), nr = std::max<size_t>(io_rids.size(), 1), ns = std::max<size_t>(io_sids.size(), 1);
+    const size_t lists = n * 8 + (2 * (n + 1) + nr + ns) * 4;
+    std::vector<unsigned char> host(lists, 0);
+    unsigned char* h8 = host.data();
+    int32_t* h4 = (int32_t*)(h8 + n * 8);
+    if (n) std::memcpy(h8, io_node.data(), n * 8);
+    std::memcpy(h4, io_roff.data(), (n + 1) * 4);
+    std::memcpy(h4 + n + 1, io_soff.data(), (n + 1) * 4);
+    if (!io_rids.empty()) std::memcpy(h4 + 2 * (n + 1), io_rids.data(), io_rids.size() * 4);
+    if (!io_sids.empty()) std::memcpy(h4 + 2 * (n + 1) + nr, io_sids.data(), io_sids.size() * 4);
+    unsigned char* d8;
+    uint8_t* flag;
+    ADJ_TRY(C, mem.get(&d8, lists));
+    ADJ_TRY(C, mem.get(&flag, (size_t)NP));
+    ADJ_TRY(C, cudaMemcpyAsync(d8, h8, lists, cudaMemcpyHostToDevice, st));
+    ADJ_TRY(C, cudaStreamSynchronize(st));  // host goes out of scope
+    ADJ_TRY(C, cudaMemsetAsync(flag, 0, (size_t)NP, st));
+    const int32_t* d4 = (const int32_t*)(d8 + n * 8);
+    IO.flag = flag;
+    IO.node = (const int64_t*)d8;
+    IO.roff = d4;
+    IO.soff = d4 + n + 1;
+    IO.rids = d4 + 2 * (n + 1);
+    IO.sids = d4 + 2 * (n + 1) + nr;
+    IO.n = (int32_t)n;
+    IO.in_band = sband_d;
+    if (n) {
+      awc::adj_mark<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(flag, IO.node, (int32_t)n);
+      ADJ_TRY(C, cudaGetLastError());
+    }
+  }
   // kernel parameters
   awc::AdjStep<T> A{};
   A.nx = (int32_t)p->nx;
@@ -1064,21 +1165,32 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
     A.zchunk = (int32_t)std::max<int64_t>(4, (nzc + chunks - 1) / chunks);
     tma_grid = dim3((unsigned)gx, (unsigned)gy, (unsigned)((nzc + A.zchunk - 1) / A.zchunk));
   }
-  // checkpoints and segment fields (gradient only)
-  const int64_t nseg = want_grad ? (nt + kchk - 1) / kchk : 0;
+  // Checkpoints and segment fields (gradient only). Where one set of all nt
+  // fields takes at most KEEP_ALL bytes (and can be had) the run is one segment:
+  // the forward run keeps every field and nothing is saved or recomputed.
+  const int64_t kask = kchk;
+  if (want_grad && (nt + 2) * fb <= KEEP_ALL) kchk = std::max<int64_t>(kchk, nt);
   int64_t band_elems = 0;
   for (int a = 0; a < p->ndim; ++a) band_elems += 2 * (V.psi_len[a] + V.xi_len[a]);
-  std::vector<T*> chk(nseg, nullptr);
+  const int64_t chk_elems = (3 * NP + band_elems + 63) / 64 * 64;
+  int64_t nseg = 0, nfield = 0;
   // segment fields: two sets, so that segment c - 1 is recomputed into one
   // while the backward steps of segment c read the other
-  const int nset = nseg > 1 ? 2 : 1;
+  int nset = 1;
+  T* arena = nullptr;  // one allocation for the saved states and the segments' fields
+  while (want_grad) {
+    nseg = (nt + kchk - 1) / kchk;
+    nset = nseg > 1 ? 2 : 1;
+    nfield = std::min<int64_t>(kchk, nt) + 2;
+    const cudaError_t e = mem.get(&arena, (nseg * chk_elems + nset * nfield * NP) * sizeof(T));
+    if (e == cudaSuccess) break;
+    if (kchk == kask) ADJ_TRY(C, e);
+    cudaGetLastError();
+    kchk = kask;
+  }
+  std::vector<T*> chk(nseg, nullptr);
   std::vector<T*> seg[2];
   if (want_grad) {
-    // one allocation for the saved states and the segments' fields
-    const int64_t chk_elems = (3 * NP + band_elems + 63) / 64 * 64;
-    const int64_t nfield = std::min<int64_t>(kchk, nt) + 2;
-    T* arena;
-    ADJ_TRY(C, mem.get(&arena, (nseg * chk_elems + nset * nfield * NP) * sizeof(T)));
     for (int64_t c = 0; c < nseg; ++c) chk[c] = arena + c * chk_elems;
     for (int b = 0; b < nset; ++b) {
       seg[b].resize(nfield);
@@ -1205,36 +1317,43 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
           A.mu_in[a][sd] = mu[a][sd][par];
           A.mu_out[a][sd] = mu[a][sd][par ^ 1];
         }
-      if (!RG.node.empty())
-        awc::adj_residuals<T><<<(unsigned)((RG.node.size() + 127) / 128), 128, 0, bs>>>(
-            A.lam, rnode_d, roff_d, rids_d, (int32_t)RG.node.size(), res_d + t * nrec);
       A.pm1 = want_grad ? seg[b][t - s] : nullptr;
       A.p0 = want_grad ? seg[b][t - s + 1] : nullptr;
       A.pp1 = want_grad ? seg[b][t - s + 2] : nullptr;
       A.grad = grad;
-      const bool fork = has_core && shell_blocks > 0;
-      if (fork) {
-        ADJ_TRY(C, cudaEventRecord(ev_fork, bs));
-        ADJ_TRY(C, cudaStreamWaitEvent(bs2, ev_fork, 0));
+      if (p->ndim == 2) {
+        IO.res = res_d + t * nrec;
+        IO.stf = stf_d + t * nsrc;
+        IO.out = sout_d ? sout_d + t * nsrc : nullptr;
+        ADJ_TRY(C, launch_2d(A, IO, want_grad, i64, bs));
+      } else {
+        if (!RG.node.empty())
+          awc::adj_residuals<T><<<(unsigned)((RG.node.size() + 127) / 128), 128, 0, bs>>>(
+              A.lam, rnode_d, roff_d, rids_d, (int32_t)RG.node.size(), res_d + t * nrec);
+        const bool fork = has_core && shell_blocks > 0;
+        if (fork) {
+          ADJ_TRY(C, cudaEventRecord(ev_fork, bs));
+          ADJ_TRY(C, cudaStreamWaitEvent(bs2, ev_fork, 0));
+        }
+        if (shell_blocks > 0)
+          launch_shell(A, want_grad, i64, shell_blocks, fork ? bs2 : bs);
+        if (has_core && use_tma) {
+          awc::adj_core_tma<T, ADJ_TY, ADJ_STAGES>
+              <<<tma_grid, dim3(32, ADJ_TY), adj_core_smem<T>(), bs>>>(
+                  map_lam[i2], map_f, map_seg[b][t - s + 1], map_lam3[i3], map_grad, A);
+        } else if (has_core) {
+          launch_core(A, want_grad, i64, core_grid, bs);
+        }
+        if (fork) {
+          ADJ_TRY(C, cudaEventRecord(ev_join, bs2));
+          ADJ_TRY(C, cudaStreamWaitEvent(bs, ev_join, 0));
+        }
+        if (nsrc > 0)
+          awc::adj_sources<T><<<1, 32, 0, bs>>>(A.lam, A.F, snode_d, sband_d, (int32_t)nsrc,
+                                                stf_d + t * nsrc, grad,
+                                                sout_d ? sout_d + t * nsrc : nullptr);
+        ADJ_TRY(C, cudaGetLastError());
       }
-      if (shell_blocks > 0)
-        launch_shell(A, p->ndim, want_grad, i64, shell_blocks, fork ? bs2 : bs);
-      if (has_core && use_tma) {
-        awc::adj_core_tma<T, ADJ_TY, ADJ_STAGES>
-            <<<tma_grid, dim3(32, ADJ_TY), adj_core_smem<T>(), bs>>>(
-                map_lam[i2], map_f, map_seg[b][t - s + 1], map_lam3[i3], map_grad, A);
-      } else if (has_core) {
-        launch_core(A, p->ndim, want_grad, i64, core_grid, bs);
-      }
-      if (fork) {
-        ADJ_TRY(C, cudaEventRecord(ev_join, bs2));
-        ADJ_TRY(C, cudaStreamWaitEvent(bs, ev_join, 0));
-      }
-      if (nsrc > 0)
-        awc::adj_sources<T><<<1, 32, 0, bs>>>(A.lam, A.F, snode_d, sband_d, (int32_t)nsrc,
-                                              stf_d + t * nsrc, grad,
-                                              sout_d ? sout_d + t * nsrc : nullptr);
-      ADJ_TRY(C, cudaGetLastError());
       std::swap(i2, i3);  // λ_{t+1} is the next step's λ_{t+2}
       par ^= 1;
     }
