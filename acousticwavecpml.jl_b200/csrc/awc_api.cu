@@ -809,13 +809,28 @@ void box_blocks(awc_plan* P) {
   for (int b = P->nbox; b < 6; ++b) P->box_blk[b + 1] = P->box_blk[b];
 }
 
-// Launch grid of the 2D kernel (x tiles of 32 from x = 0, y tiles of 8 rows
-// from y = 1) or of the 3D core kernel (x tiles of 64 from core_x, y tiles of
+// Bytes of a field from which a 2D step runs in strips (step2d_strip) instead
+// of one node per thread: us per step of the two, FP32 1000 x 1000 7.9 and 7.7,
+// 2000 x 2000 15.4 and 20.5, 5210 x 2604 48 and 89; FP64 2500 x 1500 30 and 42.
+constexpr int64_t STRIP_BYTES = 8000000;
+bool strips2d(const awc_plan* P) {
+  return (P->p.nx - 2) * (P->p.ny - 2) * (int64_t)P->esz >= STRIP_BYTES;
+}
+// Tile of a block of the 2D kernel.
+void tile2d(const awc_plan* P, int64_t* tx, int64_t* ty) {
+  *tx = strips2d(P) ? 32 * 16 / (int64_t)P->esz : 32;
+  *ty = strips2d(P) ? awc::STRIP_WARPS * awc::STRIP_R : 8;
+}
+
+// Launch grid of the 2D kernel (x tiles from x = 0, y tiles from y = 1) or of the 3D core kernel (x tiles of 64 from core_x, y tiles of
 // `by` rows from core.y0, z chunks of `zchunk` planes from core.z0).
 dim3 step_grid(const awc_plan* P) {
   const awc_problem* p = &P->p;
-  if (p->ndim == 2)
-    return dim3((unsigned)((p->nx - 2) / 32 + 1), (unsigned)((p->ny - 2 + 7) / 8), 1);
+  if (p->ndim == 2) {
+    int64_t tx, ty;
+    tile2d(P, &tx, &ty);
+    return dim3((unsigned)((p->nx - 2) / tx + 1), (unsigned)((p->ny - 2 + ty - 1) / ty), 1);
+  }
   if (!P->has_core) return dim3(0, 0, 0);
   const awc::Box& C = P->core;
   return dim3((unsigned)((C.x1 - P->core_x) / 64 + 1), (unsigned)((C.y1 - C.y0 + P->by) / P->by),
@@ -851,8 +866,10 @@ int ensure_io(awc_plan* P) {
       continue;
     }
     if (!d3) {
-      const int64_t blk = i / 32 + g.x * ((j - 1) / 8);
-      const int local = (int)(i % 32 + 32 * ((j - 1) % 8));
+      int64_t tx, ty;
+      tile2d(P, &tx, &ty);
+      const int64_t blk = i / tx + g.x * ((j - 1) / ty);
+      const int local = (int)(i % tx + tx * ((j - 1) % ty));
       ent[0].push_back({{blk, local}, make_int4(local, 0, e.sgrp, e.rgrp)});
       continue;
     }
@@ -1192,7 +1209,10 @@ int launch_step(awc_plan* P, int64_t it, const StepState& stt, cudaStream_t st) 
   }
   if (p->ndim == 2) {
     kernel_params(P, 0, S);
-    awc::step2d<T><<<step_grid(P), dim3(32, 8), 0, st>>>(S);
+    if (strips2d(P))
+      awc::step2d_strip<T><<<step_grid(P), dim3(32, awc::STRIP_WARPS), 0, st>>>(S);
+    else
+      awc::step2d<T><<<step_grid(P), dim3(32, 8), 0, st>>>(S);
   } else {
     const bool shell = P->nbox > 0, core = P->has_core;
     if (shell && core) {

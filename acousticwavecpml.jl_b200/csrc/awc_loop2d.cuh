@@ -1039,4 +1039,135 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
   }
 }
 
+// ---------------------------------------------------------------------------
+// One 2D step of a grid too large for the chip: warp w of a block owns a strip
+// of 32 vectors x R rows and issues every load of it (R + 2 pressure rows, R
+// rows of p_{t-1} and of fact, a vector per lane) before any arithmetic; x
+// neighbours come from the adjacent lanes. Bound by HBM: 16 bytes per node and
+// step in FP32. At 5210 x 2604 a step takes 47 us (4.6 TB/s) where one node per
+// thread (step2d) takes 88; strips of 1 and 4 rows 55 us, 8 warps of 4 rows 55.
+constexpr int STRIP_WARPS = 4, STRIP_R = 2;
+template <typename T>
+__global__ void __launch_bounds__(32 * STRIP_WARPS) step2d_strip(StepParams<T> P) {
+  using K = Pack<T>;
+  constexpr int V = K::V, R = STRIP_R, TX = 32 * V, TY = STRIP_WARPS * R;
+  const int lane = threadIdx.x, w = threadIdx.y;
+  const int nx = P.nx, ny = P.ny, halo = P.halo;
+  const int blk = blockIdx.x + gridDim.x * blockIdx.y;
+  if (blk == 0 && P.do_rim && P.io.nrim > 0) rim_io(P.io, P.pnew, P.it);
+  const int xw = blockIdx.x * TX, i = xw + lane * V;
+  const int j0 = 1 + blockIdx.y * TY + w * R;
+  if (j0 > ny - 2) return;  // whole warp
+  const int64_t px = P.px;
+  const T* __restrict__ pcur = P.pcur;
+  // lanes past the row's end load its last vector, rows past the grid its last
+  // rows; what they compute is not stored
+  const int64_t il = min((int64_t)i, px - V);
+  K q[R + 2], o[R], f[R];
+  T xe[R];
+#pragma unroll
+  for (int r = 0; r < R + 2; ++r) q[r] = ldg_pack<T>(pcur + il + px * min(j0 - 1 + r, ny - 1));
+  const int64_t ie = lane == 0 ? max(i - 1, 0) : min((int64_t)i + V, px - 1);
+  const bool edge = lane == 0 || lane == 31;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int64_t row = px * min(j0 + r, ny - 2);
+    o[r] = ldg_pack<T>(P.pold + il + row);
+    f[r] = ldg_pack<T>(P.fact + il + row);
+    xe[r] = edge ? __ldg(pcur + ie + row) : T(0);
+  }
+  unsigned ok = 0;
+#pragma unroll
+  for (int v = 0; v < V; ++v)
+    if (i + v >= 1 && i + v <= nx - 2) ok |= 1u << v;
+  const bool xband = (P.active[0][0] && xw <= halo) || (P.active[0][1] && xw + TX - 1 >= nx - halo - 1);
+  const bool yband = (P.active[1][0] && j0 <= halo) || (P.active[1][1] && j0 + R - 1 >= ny - halo - 1);
+  const int e0 = P.io.blk_off[blk], e1 = P.io.blk_off[blk + 1];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int j = j0 + r;
+    const K& c = q[r + 1];
+    T xm = __shfl_up_sync(0xffffffffu, c.v[V - 1], 1), xp = __shfl_down_sync(0xffffffffu, c.v[0], 1);
+    if (lane == 0) xm = xe[r];
+    if (lane == 31) xp = xe[r];
+    K nv, d2x, d2y;
+    vec_update(q[r], c, q[r + 2], o[r], f[r], xm, xp, P.inv_d2[0], P.inv_d2[1], d2x, d2y, nv);
+    if (j > ny - 2) continue;
+    if (xband || yband) {
+      // all of the row's ψ and ξ are loaded before any is used
+      T damp[V], ps[V], pm[V], xo[V];
+      K yq, ym, yx;
+      int side[V], qx[V], qy = 0;
+      bool fx[V], fy = false;
+      int by = yband ? band_of(j, ny, halo, P.first_r[1], qy, fy) : 0;
+      if (by != 0 && !P.active[1][by - 1]) by = 0;
+      const bool in = ok != 0;  // the lane's vector lies in the grid's pitched row
+      if (by != 0 && in) {
+        const BandSide<T>& B = P.band[1][by - 1];
+        yq = *reinterpret_cast<const K*>(B.psi_old + px * qy + i);
+        ym = *reinterpret_cast<const K*>(B.psi_old + px * (qy - 1) + i);
+        yx = *reinterpret_cast<const K*>(B.xi + px * (qy - 1) + i);
+      }
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        damp[v] = T(0);
+        side[v] = xband && (ok >> v & 1u) ? band_of(i + v, nx, halo, P.first_r[0], qx[v], fx[v]) : 0;
+        if (side[v] != 0 && !P.active[0][side[v] - 1]) side[v] = 0;
+        if (side[v] == 0) continue;
+        const BandSide<T>& B = P.band[0][side[v] - 1];
+        ps[v] = B.psi_old[(int64_t)(halo + 1) * j + qx[v]];
+        pm[v] = B.psi_old[(int64_t)(halo + 1) * j + qx[v] - 1];
+        xo[v] = B.xi[(int64_t)halo * j + qx[v] - 1];
+      }
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        if (side[v] == 0) continue;
+        const BandSide<T>& B = P.band[0][side[v] - 1];
+        T sq, sm, xn;
+        cpml_axis(band_coef(B, qx[v]), ps[v], pm[v], xo[v], v == 0 ? xm : c.v[v == 0 ? 0 : v - 1],
+                  c.v[v], v == V - 1 ? xp : c.v[v == V - 1 ? v : v + 1], d2x.v[v], f[r].v[v],
+                  P.inv_d[0], sq, sm, xn, damp[v]);
+        B.psi_new[(int64_t)(halo + 1) * j + qx[v]] = sq;
+        if (fx[v]) B.psi_new[(int64_t)(halo + 1) * j + qx[v] - 1] = sm;
+        B.xi[(int64_t)halo * j + qx[v] - 1] = xn;
+      }
+      if (by != 0 && in) {
+        const BandSide<T>& B = P.band[1][by - 1];
+        const BandCoef<T> cf = band_coef(B, qy);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          T sq, sm, xn;
+          cpml_axis(cf, yq.v[v], ym.v[v], yx.v[v], q[r].v[v], c.v[v], q[r + 2].v[v], d2y.v[v],
+                    f[r].v[v], P.inv_d[1], sq, sm, xn, damp[v]);
+          yq.v[v] = sq;
+          ym.v[v] = sm;
+          yx.v[v] = xn;
+        }
+        // the Dirichlet columns' entries are written too; nothing reads them
+        *reinterpret_cast<K*>(B.psi_new + px * qy + i) = yq;
+        if (fy) *reinterpret_cast<K*>(B.psi_new + px * (qy - 1) + i) = ym;
+        *reinterpret_cast<K*>(B.xi + px * (qy - 1) + i) = yx;
+      }
+#pragma unroll
+      for (int v = 0; v < V; ++v) nv.v[v] += damp[v];
+    }
+    for (int e = e0; e < e1; ++e) {
+      const int4 en = P.io.ent[e];
+      const int lx = en.x % TX - lane * V;
+      if (en.x / TX != w * R + r || lx < 0 || lx >= V) continue;
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        if (v == lx) nv.v[v] = node_io(P.io, P.it, en.z, en.w, nv.v[v]);
+    }
+    T* out = P.pnew + i + px * j;
+    if (ok == (1u << V) - 1u) {
+      *reinterpret_cast<K*>(out) = nv;
+    } else {
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        if (ok >> v & 1u) out[v] = nv.v[v];
+    }
+  }
+}
+
 }  // namespace awc

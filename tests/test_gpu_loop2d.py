@@ -3,7 +3,7 @@ chip) against the per-step kernels (shorter runs): the same arithmetic in the
 same order, so every output is bitwise the same, whatever the tiling. Sizes:
 one node wide interiors, a tile's vector width and its remainders, one tile,
 several tiles in one and both directions, more receivers than threads, bands
-that meet, sources on the Dirichlet rim and on tile edges."""
+that meet, per-step grids of one node per thread and of strips (the largest), sources on the Dirichlet rim and on tile edges."""
 import numpy as np
 import pytest
 
@@ -12,7 +12,8 @@ NT = 60
 # (nx, ny, halo, free top): ny = None is a 1D line
 GRIDS = [(3, 3, 0, False), (4, 5, 1, False), (5, 4, 1, True), (23, 19, 8, False),
          (43, 42, 20, False), (64, 67, 5, True), (131, 90, 20, True), (257, 61, 10, False),
-         (70, 401, 20, True), (409, 333, 20, False), (1030, 517, 30, True), (3, None, 0, False),
+         (70, 401, 20, True), (409, 333, 20, False), (1030, 517, 30, True),
+         (1039, 1037, 20, False), (2083, 1019, 20, True), (3, None, 0, False),
          (129, None, 20, False), (4099, None, 20, False)]
 
 
