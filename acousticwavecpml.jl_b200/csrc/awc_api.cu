@@ -2293,32 +2293,17 @@ int awc_plan_autotune(awc_plan* P, int64_t steps, float* best_ms_per_step) {
   return awc_plan_reset(P);
 }
 
-int awc_forward(awc_ctx* ctx, const awc_problem* p, const double* vel, const double* coeffs,
-                const int64_t* possrcs, const double* dt2srctf, const int64_t* posrecs,
-                double* traces, double* pfinal) {
-  if (!ctx) return set_err(nullptr, AWC_ERR_INVALID, "ctx is NULL");
-  if (p && p->ndim == 1) {
-    int rc;
-    if ((rc = validate_1d(p, &ctx->err)) ||
-        (rc = check_positions(p, possrcs, p->nsrc, "source", &ctx->err)) ||
-        (rc = check_positions(p, posrecs, p->nrec, "receiver", &ctx->err)))
-      return rc;
-    if (!vel || !coeffs) return set_err(&ctx->err, AWC_ERR_INVALID, "vel/coeffs are NULL");
-    awc_plan* P = nullptr;
-    if ((rc = awc_plan_create(ctx, p, vel, coeffs, possrcs, dt2srctf, posrecs, &P))) return rc;
-    rc = awc_plan_run(P, p->nt, 1, &ctx->last_run_ms);
-    if (!rc && traces) rc = awc_plan_traces(P, traces);
-    if (!rc && pfinal) rc = awc_plan_field(P, pfinal);
-    awc_plan_destroy(P);
-    return rc;
-  }
-  int rc = validate(p, &ctx->err);
-  if (rc) return rc;
-  if (p->nt * p->nrec > 0 && !traces) return set_err(&ctx->err, AWC_ERR_INVALID, "traces is NULL");
+namespace {
+// awc_forward for a 2D or 3D problem, or for the three-row form of a 1D one
+// (lifted1d), on a plan of the context's cache.
+int forward_cached(awc_ctx* ctx, const awc_problem* p, const double* vel, const double* coeffs,
+                   const int64_t* possrcs, const double* dt2srctf, const int64_t* posrecs,
+                   double* traces, double* pfinal, bool lifted1d) {
   // reuse a cached plan of the same shape: same buffers, same graphs
+  int rc;
   awc_plan* P = nullptr;
   for (size_t c = 0; c < ctx->cache.size(); ++c)
-    if (same_shape(ctx->cache[c]->p, *p)) {
+    if (ctx->cache[c]->is1d == lifted1d && same_shape(ctx->cache[c]->p, *p)) {
       P = ctx->cache[c];
       ctx->cache.erase(ctx->cache.begin() + c);
       break;
@@ -2340,7 +2325,8 @@ int awc_forward(awc_ctx* ctx, const awc_problem* p, const double* vel, const dou
       return rc;
     }
   } else {
-    if ((rc = forward_impl(ctx, p, vel, coeffs, possrcs, dt2srctf, posrecs, &P))) return rc;
+    if ((rc = forward_impl(ctx, p, vel, coeffs, possrcs, dt2srctf, posrecs, &P, lifted1d))) return rc;
+    P->is1d = lifted1d;
     // a new 3D shape: pick its launch shape once, on its own data
     if (p->ndim == 3 && ctx->autotune_steps > 0 && p->nt >= 100 &&
         (rc = awc_plan_autotune(P, ctx->autotune_steps, nullptr))) {
@@ -2357,6 +2343,29 @@ int awc_forward(awc_ctx* ctx, const awc_problem* p, const double* vel, const dou
   if (traces && (rc = awc_plan_traces(P, traces))) return rc;
   if (pfinal && (rc = awc_plan_field(P, pfinal))) return rc;
   return AWC_OK;
+}
+}  // namespace
+
+int awc_forward(awc_ctx* ctx, const awc_problem* p, const double* vel, const double* coeffs,
+                const int64_t* possrcs, const double* dt2srctf, const int64_t* posrecs,
+                double* traces, double* pfinal) {
+  if (!ctx) return set_err(nullptr, AWC_ERR_INVALID, "ctx is NULL");
+  if (p && p->ndim == 1) {
+    int rc;
+    if ((rc = validate_1d(p, &ctx->err)) ||
+        (rc = check_positions(p, possrcs, p->nsrc, "source", &ctx->err)) ||
+        (rc = check_positions(p, posrecs, p->nrec, "receiver", &ctx->err)))
+      return rc;
+    if (!vel || !coeffs) return set_err(&ctx->err, AWC_ERR_INVALID, "vel/coeffs are NULL");
+    Lifted L;
+    lift_1d(p, vel, coeffs, possrcs, posrecs, &L);
+    return forward_cached(ctx, &L.p, L.vel.data(), L.coeffs.data(), L.possrcs.data(), dt2srctf,
+                          L.posrecs.data(), traces, pfinal, true);
+  }
+  int rc = validate(p, &ctx->err);
+  if (rc) return rc;
+  if (p->nt * p->nrec > 0 && !traces) return set_err(&ctx->err, AWC_ERR_INVALID, "traces is NULL");
+  return forward_cached(ctx, p, vel, coeffs, possrcs, dt2srctf, posrecs, traces, pfinal, false);
 }
 
 int awc_forward_decomposed(awc_ctx* const* ctxs, int32_t nsub, const awc_problem* p,
