@@ -57,81 +57,16 @@ Loop2D::~Loop2D() {
 
 namespace {
 
-// Relative cost of one row of one vector: a plain one, and what an x band and
-// a y band add. The bands' share is their instructions and, more, their
-// longer dependent chains; of the values tried (x 70 to 220, y 50 to 100)
-// these gave the shortest steps at 1573 x 787 and 1088 x 532 together.
-constexpr int kRow = 45, kRowX = 150, kRowY = 80;
+// Relative cost of one vector of nodes: a plain one, and what an x band and a y
+// band add (instructions, counted from the operations).
+constexpr int kRow = 45, kRowX = 110, kRowY = 90;
 
 // A tile's rows: y-band rows, plain rows, y-band rows.
 struct Rows {
   int n[3] = {};
+  int all() const { return n[0] + n[1] + n[2]; }
   bool operator==(const Rows& o) const { return n[0] == o.n[0] && n[1] == o.n[1] && n[2] == o.n[2]; }
 };
-// Rows per thread of a column class (columns with x-band nodes or without) in
-// plain or y-band rows: as many as `budget` pays for, at least one.
-int run_rows(int budget, bool xcol, bool y) {
-  const int c = kRow + (xcol ? kRowX : 0) + (y ? kRowY : 0);
-  return std::max(1, std::min(LOOP_ROWS, budget / c));
-}
-
-// The threads of a tile of cw vector columns, nvx of them with x-band nodes:
-// the smallest budget per thread that needs at most LOOP_NT threads. A band
-// row costs several plain ones, so threads of the bands get fewer rows.
-struct Cut {
-  int threads = 0, rows = 0, budget = 0, nyt = 0, yrows = 0;
-  double work = 0;  // cost of all rows of all vectors
-  bool ok = false;
-};
-Cut cut_tile(const Rows& y, int cw, int nvx) {
-  Cut best;
-  auto runs = [&](int budget, bool xcol, bool yband) {
-    const int k = run_rows(budget, xcol, yband);
-    return yband ? (y.n[0] + k - 1) / k + (y.n[2] + k - 1) / k : (y.n[1] + k - 1) / k;
-  };
-  auto count = [&](int budget) {
-    return (cw - nvx) * (runs(budget, false, false) + runs(budget, false, true)) +
-           nvx * (runs(budget, true, false) + runs(budget, true, true));
-  };
-  int lo = kRow, hi = LOOP_ROWS * (kRow + kRowX + kRowY);
-  if (count(hi) > LOOP_NT) return best;
-  while (lo < hi) {
-    const int mid = (lo + hi) / 2;
-    if (count(mid) <= LOOP_NT)
-      hi = mid;
-    else
-      lo = mid + 1;
-  }
-  best.ok = true;
-  best.budget = lo;
-  best.threads = count(lo);
-  for (int c = 0; c < 2; ++c) {
-    const int cols = c ? nvx : cw - nvx;
-    if (cols == 0) continue;
-    best.nyt += cols * runs(lo, c == 1, true);
-    const int ky = run_rows(lo, c == 1, true), k = run_rows(lo, c == 1, false);
-    if (y.n[1]) best.rows = std::max(best.rows, std::min(k, y.n[1]));
-    const int most = std::min(ky, std::max(y.n[0], y.n[2]));
-    best.rows = std::max(best.rows, most);
-    best.yrows = std::max(best.yrows, most);
-    best.work += (double)cols * (y.n[1] * (kRow + (c ? kRowX : 0)) +
-                                 (y.n[0] + y.n[2]) * (kRow + kRowY + (c ? kRowX : 0)));
-  }
-  return best;
-}
-
-// Estimated cycles of one step of a tile: the longer of a thread's dependent
-// chain and the block's issue, and the trip of the edges, which a tile with
-// edge items mostly hides. Fitted to measured steps of single tiles (128 x
-// 32, 64 and 128 nodes: 0.67, 1.1 and 1.9 us) and of pairs (0.8 us more).
-double step_cost(const Cut& c, bool exchange, int items) {
-  const double warps = (c.threads + 31) / 32;
-  const double chain = 5.5 * (100.0 + c.budget);
-  const double issue = 1.7 * (warps * 100.0 + c.work / 32.0) / 4.0;
-  const double edge = exchange ? (c.rows >= LOOP_EARLY_R ? 1200.0 + 8.0 * items : 1500.0 + 2.0 * items) : 0.0;
-  return 300.0 + std::max(chain, issue) + edge;
-}
-
 // The kinds of rows y0 .. y0 + h - 1 of a shot.
 Rows tile_rows(int y0, int h, int64_t ny, int halo, const int32_t* active) {
   const BandSlots b = band_slots(y0, h, 1, (int)ny, halo, first_right(ny, halo), active[0] != 0, active[1] != 0);
@@ -140,6 +75,32 @@ Rows tile_rows(int y0, int h, int64_t ny, int halo, const int32_t* active) {
   r.n[2] = b.nb;
   r.n[1] = h - b.na - b.nb;
   return r;
+}
+// Rows per thread of a tile of cw vector columns and h rows: the fewest that
+// need at most LOOP_NT threads (0: more than LOOP_ROWS).
+int thread_rows(int cw, int h) {
+  const int runs = LOOP_NT / cw;
+  if (runs == 0) return 0;
+  const int k = (h + runs - 1) / runs;
+  return k <= LOOP_ROWS ? k : 0;
+}
+int band_vectors(int cw, int nvx, const Rows& y) { return nvx * y.all() + (y.n[0] + y.n[2]) * (cw - nvx); }
+
+// Estimated cycles of one step of a tile. A plain row costs a warp about 50
+// instructions, 5.5 cycles each when the block has few warps to hide them and
+// 1.7 of an issue slot when it has many; a round of band vectors (one per
+// thread) 800 to 1600 cycles. Edges sent after the update are waited for, 1700
+// cycles; sent before it they cost a round themselves.
+double step_cost(int cw, int nvx, const Rows& y, bool exchange) {
+  const int h = y.all(), k = thread_rows(cw, h), nb = band_vectors(cw, nvx, y);
+  const int threads = (cw * ((h + k - 1) / k) + 31) / 32 * 32;
+  const double chain = 5.5 * (60.0 + 50.0 * k);
+  const double issue = 1.7 / 4.0 * (threads / 32 * 60.0 + cw * (double)h / 32.0 * 50.0);
+  const double rounds = (nb + threads - 1) / threads;
+  const double band = nb == 0 ? 0.0 : k == 1 ? 800.0 : 150.0 + 1100.0 * rounds;
+  const bool early = k >= LOOP_EARLY_R && 2 * (cw + h) <= threads;
+  const double edge = !exchange ? 0.0 : (early ? 1300.0 : 1900.0) + 2.0 * cw + 4.0 * h;
+  return 300.0 + std::max(chain, issue) + band + edge;
 }
 
 // Cuts n units of the given costs into `parts` consecutive parts of about equal
@@ -177,27 +138,32 @@ std::vector<int> row_costs(int64_t ny, int halo, const int32_t* active) {
   return c;
 }
 
-// Byte offsets of a tile's shared memory; returns the total.
+// Byte offsets of a tile's shared memory (`rows`: the most rows per thread of
+// its launch); returns the total.
 template <typename T>
-int tile_smem(LoopTile& L, int rows, int yrows) {
+int tile_smem(LoopTile& L, int rows) {
   constexpr int V = 16 / (int)sizeof(T);
-  int o = 0;
+  int64_t o = 0;
   auto take = [&](int64_t bytes) {
-    const int at = o;
-    o += (int)((bytes + 15) / 16 * 16);
-    return at;
+    const int64_t at = o;
+    o += (bytes + 15) / 16 * 16;
+    return (int32_t)at;
   };
   const int64_t field = (int64_t)(L.h + rows + 1) * (L.w + 2 * V) * (int64_t)sizeof(T);
+  const int64_t nb = L.nband, nx = (int64_t)L.nvx * L.h, nyv = (int64_t)(L.ny0 + L.ny1) * (L.w / V);
   L.f[0] = take(field);
   L.f[1] = take(field);
   L.cx = take(4 * (L.w + V) * (int64_t)sizeof(T));
   L.cy = take(4 * ((L.h + V) / V * V) * (int64_t)sizeof(T));
-  L.px = take((int64_t)L.nvx * L.h * 16);
-  L.xx = take((int64_t)L.nvx * L.h * 16);
-  L.px0 = take((int64_t)L.nvx * L.h * (int64_t)sizeof(T));
-  L.py = take((int64_t)L.nyt * (yrows + 1) * 16);
-  L.xy = take((int64_t)L.nyt * yrows * 16);
-  return o;
+  L.bt = take(4 * nb);
+  L.bf = take(16 * nb);
+  L.px = take(16 * nx);
+  L.px0 = take((int64_t)sizeof(T) * nx);
+  L.xx = take(16 * nx);
+  L.ylo = take(16 * nyv);
+  L.yhi = take(16 * nyv);
+  L.xy = take(16 * nyv);
+  return (int)std::min<int64_t>(o, 1 << 30);
 }
 
 }  // namespace
@@ -246,15 +212,19 @@ std::vector<Loop2D::Tiling> Loop2D::tilings(const Shape& s, bool f64, int max_ti
       for (const auto& c : cols)
         for (const auto& y : ys) {
           if (!ok) break;
-          const Cut cut = cut_tile(y, c.first, c.second);
+          if (thread_rows(c.first, y.all()) == 0) {
+            ok = false;
+            break;
+          }
           LoopTile L{};
           L.w = c.first * V;
-          L.h = y.n[0] + y.n[1] + y.n[2];
+          L.h = y.all();
           L.nvx = c.second;
-          L.nyt = cut.nyt;
-          const int smem = f64 ? tile_smem<double>(L, LOOP_ROWS, cut.yrows) : tile_smem<float>(L, LOOP_ROWS, cut.yrows);
-          ok = cut.ok && smem <= kMaxSmem;
-          t.cost = std::max(t.cost, step_cost(cut, tx * ty > 1, 2 * (c.first + L.h)));
+          L.ny0 = y.n[0];
+          L.ny1 = y.n[2];
+          L.nband = band_vectors(c.first, c.second, y);
+          ok = (f64 ? tile_smem<double>(L, LOOP_ROWS) : tile_smem<float>(L, LOOP_ROWS)) <= kMaxSmem;
+          t.cost = std::max(t.cost, step_cost(c.first, c.second, y, tx * ty > 1));
         }
       Tiling& slot = best[tx * ty];
       if (ok && t.cost < slot.cost) {
@@ -344,15 +314,13 @@ bool Loop2D::plan_waves(const awc_ctx* C) {
   return true;
 }
 
-// The tiles of every wave with their thread and item tables (uploaded once per
-// layout), mailbox sizes and launch shapes.
+// The tiles of every wave with their edge items (uploaded once per layout),
+// mailbox sizes and launch shapes.
 template <typename T>
 int Loop2D::lay_out(awc_ctx* C) {
   constexpr int V = 16 / (int)sizeof(T), WPV = (int)sizeof(T) / 4;
-  std::vector<LoopThread> threads;
-  std::vector<LoopItem> items;
+  std::vector<LoopEdge> edges;
   tiles_.clear();
-  owners_.clear();
   int hm = 0, wm = 0;
   int64_t most = 0;
   int64_t count = 0;
@@ -374,24 +342,17 @@ int Loop2D::lay_out(awc_ctx* C) {
   mail_stride_ = 2 * ((words + 31) / 32 * 32);
   for (Wave& wv : waves_) {
     const int oL = 0, oR = wv.hmax * WPV, oU = 2 * wv.hmax * WPV, oD = (2 * wv.hmax + wv.wmax) * WPV;
-    struct Built {
-      LoopTile L;
-      Cut cut;
-      Rows y;
-    };
-    std::vector<Built> built;
+    const size_t begin = tiles_.size();
     wv.R = 1;
     wv.first.clear();
     for (size_t q = 0; q < wv.shots.size(); ++q) {
       const Shape& sh = shapes_[wv.shots[q]];
       const Tiling& t = wv.tiling[q];
-      wv.first.push_back((int)built.size());
-      const int first = (int)built.size();
+      const int first = (int)(tiles_.size() - begin);
+      wv.first.push_back(first);
       for (int ty = 0; ty < t.ty; ++ty)
         for (int tx = 0; tx < t.tx; ++tx) {
-          Built b;
-          LoopTile& L = b.L;
-          L = LoopTile{};
+          LoopTile L{};
           L.shot = wv.shots[q];
           L.x0 = t.xb[tx] * V;
           L.w = (t.xb[tx + 1] - t.xb[tx]) * V;
@@ -404,98 +365,52 @@ int Loop2D::lay_out(awc_ctx* C) {
           L.nbr[3] = ty + 1 < t.ty ? me + t.tx : -1;
           const BandSlots bx = band_slots(L.x0, L.w, V, (int)sh.nx, sh.halo, first_right(sh.nx, sh.halo),
                                           sh.active[0][0] != 0, sh.active[0][1] != 0);
+          const Rows y = tile_rows(L.y0, L.h, sh.ny, sh.halo, sh.active[1]);
           L.nvx = bx.na + bx.nb;
-          b.y = tile_rows(L.y0, L.h, sh.ny, sh.halo, sh.active[1]);
-          b.cut = cut_tile(b.y, L.w / V, L.nvx);
-          L.nyt = b.cut.nyt;
-          wv.R = std::max(wv.R, b.cut.rows);
-          built.push_back(std::move(b));
+          L.ny0 = y.n[0];
+          L.ny1 = y.n[2];
+          L.nband = band_vectors(L.w / V, L.nvx, y);
+          L.rows = thread_rows(L.w / V, L.h);
+          wv.R = std::max(wv.R, L.rows);
+          tiles_.push_back(L);
         }
     }
     if (wv.R == 7) wv.R = 8;  // the kernel's instances
     wv.threads = 32;
     wv.smem = 0;
-    for (Built& b : built) {
-      LoopTile& L = b.L;
+    for (size_t k = begin; k < tiles_.size(); ++k) {
+      const LoopTile& L = tiles_[k];
+      wv.threads = std::max(wv.threads, (L.w / V * ((L.h + L.rows - 1) / L.rows) + 31) / 32 * 32);
+    }
+    for (size_t k = begin; k < tiles_.size(); ++k) {
+      LoopTile& L = tiles_[k];
       const Shape& sh = shapes_[L.shot];
-      wv.smem = std::max(wv.smem, tile_smem<T>(L, wv.R, b.cut.yrows));
+      wv.smem = std::max(wv.smem, tile_smem<T>(L, wv.R));
       const int cw = L.w / V;
-      const BandSlots bx = band_slots(L.x0, L.w, V, (int)sh.nx, sh.halo, first_right(sh.nx, sh.halo),
-                                      sh.active[0][0] != 0, sh.active[0][1] != 0);
-      L.thr0 = (int)threads.size();
-      L.nthr = b.cut.threads;
-      wv.threads = std::max(wv.threads, (L.nthr + 31) / 32 * 32);
-      // x-band columns first, so that a warp's lanes mostly agree on whether
-      // they run the band code; within a class, run by run
-      int ys = 0;
-      std::vector<int> thread_of((size_t)cw * L.h);
-      for (int c = 1; c >= 0; --c) {
-        const int cols = c ? L.nvx : cw - L.nvx;
-        if (cols == 0) continue;
-        for (int seg = 0, at = 0; seg < 3; at += b.y.n[seg++]) {
-          const bool y = seg != 1;
-          const int k = run_rows(b.cut.budget, c == 1, y);
-          for (int r0 = at; r0 < at + b.y.n[seg]; r0 += k) {
-            const int n = std::min(k, at + b.y.n[seg] - r0);
-            for (int u = 0; u < cols; ++u) {
-              const int col = c ? (u < bx.na ? bx.a0 + u : bx.b0 + u - bx.na) : bx.other(u);
-              for (int r = r0; r < r0 + n; ++r)
-                thread_of[(size_t)r * cw + col] = (int)threads.size() - L.thr0;
-              threads.push_back(LoopThread{(int16_t)col, (int16_t)r0, (int16_t)n, (int16_t)(y ? ys++ : -1)});
-            }
-          }
-        }
-      }
-      // edge items, where the update is long enough to hide the trip
-      L.item0 = (int)items.size();
+      // edge items, where the update is long enough to hide the trip: at most
+      // one per thread
       const int n = (L.nbr[2] >= 0 ? cw : 0) + (L.nbr[3] >= 0 ? cw : 0) + (L.nbr[0] >= 0 ? L.h : 0) +
                     (L.nbr[1] >= 0 ? L.h : 0);
-      L.nitem = wv.R >= LOOP_EARLY_R ? n : 0;
-      auto item = [&](int row, int col, int nbr, int at, int what) {
-        LoopItem m{};
-        m.rc = row << 16 | col * V;
-        m.mail = (int)(nbr * mail_stride_) + at;
-        m.flag = what;
-        const int sx = bx.slot(col);
-        if (sx >= 0) {
-          m.flag |= 4 | sx << 16;
-          const int fr = first_right(sh.nx, sh.halo);
-          for (int v = 0; v < V; ++v) {
-            const int i = L.x0 + col * V + v;
-            if ((sh.active[0][0] && i >= 1 && i <= sh.halo && i <= sh.nx - 2) ||
-                (sh.active[0][1] && i >= fr && i <= sh.nx - 2))
-              m.flag |= 256 << v;
-          }
-        }
-        if (row < b.y.n[0] || row >= b.y.n[0] + b.y.n[1]) {
-          const LoopThread& th = threads[L.thr0 + thread_of[(size_t)row * cw + col]];
-          m.flag |= 8;
-          m.py = th.ys + (row - th.r0) * L.nyt;
-          m.xy = m.py;
-        }
-        items.push_back(m);
+      L.edge0 = (int)edges.size();
+      if (wv.R < LOOP_EARLY_R || n > wv.threads) continue;
+      L.nedge = n;
+      const BandVecs bv{band_slots(L.x0, L.w, V, (int)sh.nx, sh.halo, first_right(sh.nx, sh.halo),
+                                   sh.active[0][0] != 0, sh.active[0][1] != 0),
+                        cw, L.h, L.ny0, L.ny1};
+      auto item = [&](int row, int c, int nbr, int at, int what) {
+        edges.push_back(LoopEdge{row << 16 | c, (int)(nbr * mail_stride_) + at, bv.index(row, c), what});
       };
-      if (L.nitem) {
-        for (int c = 0; L.nbr[2] >= 0 && c < cw; ++c) item(0, c, L.nbr[2], oD + c * V * WPV, 0);
-        for (int c = 0; L.nbr[3] >= 0 && c < cw; ++c) item(L.h - 1, c, L.nbr[3], oU + c * V * WPV, 0);
-        for (int r = 0; L.nbr[0] >= 0 && r < L.h; ++r) item(r, 0, L.nbr[0], oR + r * WPV, 1);
-        for (int r = 0; L.nbr[1] >= 0 && r < L.h; ++r) item(r, cw - 1, L.nbr[1], oL + r * WPV, 2);
-      }
-      owners_.push_back(std::move(thread_of));
-      tiles_.push_back(L);
+      for (int c = 0; L.nbr[2] >= 0 && c < cw; ++c) item(0, c, L.nbr[2], oD + c * V * WPV, 0);
+      for (int c = 0; L.nbr[3] >= 0 && c < cw; ++c) item(L.h - 1, c, L.nbr[3], oU + c * V * WPV, 0);
+      for (int r = 0; L.nbr[0] >= 0 && r < L.h; ++r) item(r, 0, L.nbr[0], oR + r * WPV, 1);
+      for (int r = 0; L.nbr[1] >= 0 && r < L.h; ++r) item(r, cw - 1, L.nbr[1], oL + r * WPV, 2);
     }
-    for (int64_t k = wv.tile0; k < (int64_t)tiles_.size(); ++k)
-      if (tiles_[k].nitem > wv.threads) tiles_[k].nitem = 0;  // one item per thread
   }
-  const size_t tb = (threads.size() * sizeof(LoopThread) + 255) / 256 * 256, ib = items.size() * sizeof(LoopItem);
+  const size_t eb = edges.size() * sizeof(LoopEdge);
   if (table_) cudaFree(table_);
   table_ = nullptr;
-  LOOP_TRY(C, cudaMalloc(&table_, tb + ib + 16));
-  o_items_ = tb;
-  LOOP_TRY(C, cudaMemcpyAsync(table_, threads.data(), threads.size() * sizeof(LoopThread),
-                              cudaMemcpyHostToDevice, C->stream));
-  if (ib)
-    LOOP_TRY(C, cudaMemcpyAsync((char*)table_ + tb, items.data(), ib, cudaMemcpyHostToDevice, C->stream));
+  LOOP_TRY(C, cudaMalloc(&table_, eb + 16));
+  if (eb) LOOP_TRY(C, cudaMemcpyAsync(table_, edges.data(), eb, cudaMemcpyHostToDevice, C->stream));
   if (mail_) cudaFree(mail_);
   mail_ = nullptr;
   mail_bytes_ = (size_t)(mail_stride_ * most) * 8;
@@ -569,8 +484,8 @@ int Loop2D::upload(awc_ctx* C, const std::vector<LoopShotHost>& shots) {
         const bool in = i >= 1 && i <= H.nx - 2 && j >= 1 && j <= H.ny - 2;
         if (e.sgrp >= 0) {
           // a source on an edge node: this tile sends its edges after the update
-          if (r == 0 || r == L.h - 1 || c == 0 || c == L.w - 1) L.nitem = 0;
-          ts[n].push_back(LoopSrc{owners_[base + n][(size_t)r * (L.w / V) + c / V], cell, e.sgrp,
+          if (r == 0 || r == L.h - 1 || c == 0 || c == L.w - 1) L.nedge = 0;
+          ts[n].push_back(LoopSrc{r / L.rows * (L.w / V) + c / V, cell, e.sgrp,
                                   in ? (int64_t)-1 : e.node});
         }
         if (e.rgrp >= 0)
@@ -651,8 +566,7 @@ int Loop2D::launch(awc_ctx* C, const LoopSpan& span, cudaStream_t st) {
     LoopRun<T> Q{};
     const unsigned char* b = (const unsigned char*)blob_;
     Q.tiles = (const LoopTile*)b + wv.tile0;
-    Q.threads = (const LoopThread*)table_;
-    Q.items = (const LoopItem*)((const char*)table_ + o_items_);
+    Q.edges = (const LoopEdge*)table_;
     Q.shots = (const LoopShot<T>*)(b + o_shots_);
     Q.srcs = (const LoopSrc*)(b + o_srcs_);
     Q.recs = (const LoopRec*)(b + o_recs_);

@@ -53,34 +53,31 @@ struct LoopSrc {
 
 // One tile: columns [x0, x0 + w) (x0 and w multiples of a 16-byte vector; the
 // Dirichlet columns i = 0 and nx - 1 belong to the outer tiles and are
-// masked), interior rows [y0, y0 + h). Built on the host with the lists of
-// its threads and edge items and its shared-memory layout.
+// masked), interior rows [y0, y0 + h). Built on the host with the list of its
+// edge items and its shared-memory layout.
 struct LoopTile {
   int32_t shot;
   int32_t x0, y0, w, h;
   int32_t nbr[4];          // tile index of the left, right, upper, lower neighbour, or -1
-  int32_t thr0, nthr;      // threads that own nodes
-  int32_t item0, nitem;    // edge items, 0 when the edges are sent after the update
+  int32_t rows;            // rows of a thread (the last run of a column may have fewer)
+  int32_t edge0, nedge;    // edge items; none when the edges are sent after the update
   int32_t src[2], rec[2];  // ranges in the entry lists
-  int32_t nvx, nyt;        // vector columns with x-band nodes, threads with y-band rows
+  int32_t nvx;             // vector columns with x-band nodes
+  int32_t ny0, ny1;        // y-band rows at the tile's top and bottom
+  int32_t nband;           // vectors with CPML work: nvx * h of the x-band columns, row by
+                           // row, then those of the y-band rows in the other columns
   // byte offsets in shared memory: the two fields; the coefficient tables
-  // 4 x (w + V) and 4 x (h + V); x bands: ψ on the right faces, ξ (vectors of
-  // each row), ψ on the left face (scalars); y bands: ψ on a thread's faces, ξ
-  int32_t f[2], cx, cy, px, xx, px0, py, xy;
-};
-// Thread `tid` of a tile owns the V columns of vector cv in rows
-// [r0, r0 + nrow); ys: its number among the threads with y-band rows, or -1.
-struct LoopThread {
-  int16_t cv, r0, nrow, ys;
+  // 4 x (w + V) and 4 x (h + V); per band vector its row << 16 | column, fact, and
+  // in the x-band ones ψ
+  // on the nodes' right faces, on the vector's left face (scalar) and ξ; per
+  // vector of a y-band row ψ on its upper and lower faces and ξ
+  int32_t f[2], cx, cy, bt, bf, px, px0, xx, ylo, yhi, xy;
 };
 // An edge item: one vector of the tile whose new value (all of it, or its
-// first or last node) goes to mailbox word `mail`. rc: row << 16 | column.
-// py: index of its ψ on the upper face among the y states (the lower face
-// follows nyt further), xy: of its ξ. flag: bits 0-1 what is sent (0 all, 1
-// first, 2 last), 4 x band, 8 y band, 256 << v node v in an x band,
-// x-band column << 16.
-struct LoopItem {
-  int32_t rc, mail, py, xy, flag;
+// first or last node) goes to mailbox word `mail`. rc: row << 16 | vector.
+// band: its number among the band vectors, or -1. what: 0 all, 1 first, 2 last.
+struct LoopEdge {
+  int32_t rc, mail, band, what;
 };
 
 template <typename T>
@@ -110,8 +107,7 @@ struct LoopShot {
 template <typename T>
 struct LoopRun {
   const LoopTile* tiles;
-  const LoopThread* threads;
-  const LoopItem* items;
+  const LoopEdge* edges;
   const LoopShot<T>* shots;
   const LoopSrc* srcs;
   const LoopRec* recs;
@@ -167,6 +163,37 @@ __host__ __device__ inline BandSlots band_slots(int first, int count, int unit, 
   }
   return s;
 }
+
+// Band vector number k of a tile of cw vector columns and h rows: its row and
+// column, and back (-1: no CPML work).
+struct BandVecs {
+  BandSlots bx;
+  int cw, h, ny0, ny1;
+  __host__ __device__ int nvx() const { return bx.na + bx.nb; }
+  __host__ __device__ int count() const { return nvx() * h + (ny0 + ny1) * (cw - nvx()); }
+  __host__ __device__ int yrow(int row) const {  // number of a y-band row, or -1
+    return row < ny0 ? row : row >= h - ny1 ? ny0 + row - (h - ny1) : -1;
+  }
+  __host__ __device__ void at(int k, int& row, int& cv) const {
+    const int n = nvx();
+    if (k < n * h) {
+      row = k / n;
+      const int q = k - row * n;
+      cv = q < bx.na ? bx.a0 + q : bx.b0 + q - bx.na;
+    } else {
+      const int m = cw - n, y = (k - n * h) / m;
+      row = y < ny0 ? y : h - ny1 + y - ny0;
+      cv = bx.other(k - n * h - y * m);
+    }
+  }
+  __host__ __device__ int index(int row, int cv) const {
+    const int n = nvx(), s = bx.slot(cv), y = yrow(row);
+    if (s >= 0) return row * n + s;
+    if (y < 0) return -1;
+    const int before = (cv >= bx.a0 + bx.na ? bx.na : 0) + (cv >= bx.b0 + bx.nb ? bx.nb : 0);
+    return n * h + y * (cw - n) + cv - before;
+  }
+};
 
 template <typename T>
 struct alignas(16) Pack {
@@ -446,29 +473,29 @@ __device__ __forceinline__ void vec_xband(uint32_t ca, int cs, const Pack<T>& c,
 }
 
 // R: the most rows a thread of the launch owns. A vector is 16 bytes: 4 floats
-// or 2 doubles.
+// or 2 doubles. Thread t owns the V columns of vector t % cw in the `rows` rows
+// from (t / cw) rows on.
 template <typename T, int R>
 __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ LoopRun<T> Q) {
   constexpr int V = 16 / (int)sizeof(T);
   constexpr int WPV = (int)sizeof(T) / 4;  // mailbox words per value
+  constexpr int ES = (int)sizeof(T);
   using P = Pack<T>;
   extern __shared__ __align__(128) unsigned char smem[];
   const LoopTile& tl = Q.tiles[blockIdx.x];
   const LoopShot<T>& S = Q.shots[tl.shot];
-  const int tid = threadIdx.x;
-  const int nthr = blockDim.x;
+  const int tid = threadIdx.x, nthr = blockDim.x;
   const int w = tl.w, h = tl.h, x0 = tl.x0, y0 = tl.y0;
   const int nx = S.nx, ny = S.ny, halo = S.halo;
   const int64_t px = S.px;
-  const int cw = w / V;
-  const BandSlots bx = band_slots(x0, w, V, nx, halo, S.first_r[0], S.active[0][0] != 0,
-                                  S.active[0][1] != 0);
-  const int nvx = tl.nvx, nyt = tl.nyt;
-  const int pitch = w + 2 * V;
+  const int cw = w / V, pitch = w + 2 * V;
+  const BandVecs bv{band_slots(x0, w, V, nx, halo, S.first_r[0], S.active[0][0] != 0,
+                               S.active[0][1] != 0),
+                    cw, h, tl.ny0, tl.ny1};
+  const int nband = tl.nband, nxv = tl.nvx * h;
   // cur and nxt: the fields of p_t and of p_{t-1}, which becomes p_{t+1}
   const uint32_t sb = smem_u32(smem);
   uint32_t cur = sb + tl.f[0], nxt = sb + tl.f[1];
-  constexpr int ES = (int)sizeof(T);
   // coefficient tables: face c of an axis lies between the tile's nodes c - 1
   // and c; node c of a band uses faces c and c + 1. Zero outside the bands.
   T* const cx = reinterpret_cast<T*>(smem + tl.cx);
@@ -476,6 +503,9 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
   const int cxs = w + V;  // {bKh, ah} of the faces, {bK, a} of the nodes
   T* const cy = reinterpret_cast<T*>(smem + tl.cy);
   const int cys = (h + V) / V * V;
+  const uint32_t bf_a = sb + tl.bf, px_a = sb + tl.px, px0_a = sb + tl.px0, xx_a = sb + tl.xx;
+  const int bt_o = tl.bt;
+  const uint32_t ylo_a = sb + tl.ylo, yhi_a = sb + tl.yhi, xy_a = sb + tl.xy;
   // ---- load: coefficient tables, fields with their ring, band state --------
   auto table = [&](int a, int c, int g0, int n, T* tab, int stride) {
     const int hl = halo < n - 2 ? halo : n - 2;
@@ -519,47 +549,26 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
       sts(nxt + e * ES, vo);
     }
   }
-  const bool live = tid < tl.nthr;
-  const LoopThread me = Q.threads[tl.thr0 + (live ? tid : 0)];  // idle threads shadow the first
-  const int cv = me.cv, r0 = me.r0, nrow = live ? me.nrow : 0;
-  const int i0 = x0 + cv * V;
-  // which of the vector's nodes are updated
-  unsigned okm = 0;
+  // which nodes of vector cv are updated, which lie in an active x band
+  auto ok_of = [&](int c) {
+    unsigned m = 0;
 #pragma unroll
-  for (int v = 0; v < V; ++v)
-    if (i0 + v >= 1 && i0 + v <= nx - 2) okm |= 1u << v;
-  const bool full = okm == (1u << V) - 1u;
-  const int xs = live ? bx.slot(cv) : -1, ys = live ? me.ys : -1;
-  unsigned xin = 0;  // nodes of the vector in an active x band
-  if (xs >= 0) {
+    for (int v = 0; v < V; ++v)
+      if (x0 + c * V + v >= 1 && x0 + c * V + v <= nx - 2) m |= 1u << v;
+    return m;
+  };
+  const int xl = S.active[0][0] ? min(halo, nx - 2) : 0, xr = S.active[0][1] ? S.first_r[0] : nx;
+  auto xin_of = [&](int c) {
+    unsigned m = 0;
 #pragma unroll
     for (int v = 0; v < V; ++v) {
-      const int i = i0 + v;
-      if ((S.active[0][0] && i >= 1 && i <= halo && i <= nx - 2) ||
-          (S.active[0][1] && i >= S.first_r[0] && i <= nx - 2))
-        xin |= 1u << v;
+      const int i = x0 + c * V + v;
+      if ((i >= 1 && i <= xl) || (i >= xr && i <= nx - 2)) m |= 1u << v;
     }
-  }
-  unsigned yin = 0, yfc = 0;  // rows of the group in an active y band, faces they use
-  if (ys >= 0) {
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int j = y0 + r0 + r;
-      if (r < nrow && ((S.active[1][0] && j >= 1 && j <= halo) ||
-                       (S.active[1][1] && j >= S.first_r[1] && j <= ny - 2))) {
-        yin |= 1u << r;
-        yfc |= 3u << r;
-      }
-    }
-  }
-  // the thread's x-band state of row r: row r0 + r of its column
-  const int xv = (r0 * nvx + (xs >= 0 ? xs : 0)) * 16, dxv = nvx * 16, dx0 = nvx * ES;
-  const uint32_t px_a = sb + tl.px + xv, xx_a = sb + tl.xx + xv, px0_a = sb + tl.px0 + xv / 16 * ES;
-  // its y-band state: faces 0 .. nrow and rows
-  const int yv = (ys >= 0 ? ys : 0) * 16, dyv = nyt * 16;
-  const uint32_t py_a = sb + tl.py + yv, xy_a = sb + tl.xy + yv;
-  // ψ and ξ entry of node c: side (0, 1) and q; the array index is formed per axis
-  auto side_q = [&](int a, int c, int n, int& q) {
+    return m;
+  };
+  // side (0, 1) and entry q of a band node c of an axis of n nodes
+  auto side_q = [&](int c, int n, int& q) {
     if (c <= halo) {
       q = c;
       return 0;
@@ -567,64 +576,62 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
     q = c - (n - halo - 2);
     return 1;
   };
-  if (xs >= 0) {
+  for (int k = tid; k < nband; k += nthr) {
+    int row, c;
+    bv.at(k, row, c);
+    reinterpret_cast<int*>(smem + tl.bt)[k] = row << 16 | c;
+    const int i = x0 + c * V, j = y0 + row;
+    const unsigned ok = ok_of(c);
+    P f = splat(T(0));
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      if (r >= nrow) break;
-      const int j = y0 + r0 + r;
-      P ps, xi;
+    for (int v = 0; v < V; ++v)
+      if (ok >> v & 1u) f.v[v] = S.fact[i + v + px * j];
+    sts(bf_a + k * 16, f);
+    if (k < nxv) {
+      const unsigned xin = xin_of(c);
+      P ps = splat(T(0)), xi = splat(T(0));
       T p0 = 0;
-#pragma unroll
-      for (int v = 0; v < V; ++v) ps.v[v] = xi.v[v] = T(0);
 #pragma unroll
       for (int v = 0; v < V; ++v) {
         if (!(xin >> v & 1u)) continue;
         int q;
-        const int sd = side_q(0, i0 + v, nx, q);
+        const int sd = side_q(i + v, nx, q);
         const T* psi = S.psi[0][sd][Q.par_in] + (int64_t)(halo + 1) * j;
         ps.v[v] = psi[q];
         (v == 0 ? p0 : ps.v[v == 0 ? 0 : v - 1]) = psi[q - 1];
         xi.v[v] = S.band[0][sd].xi[(int64_t)halo * j + q - 1];
       }
-      sts(px_a + r * dxv, ps);
-      sts(xx_a + r * dxv, xi);
-      sts(px0_a + r * dx0, p0);
+      sts(px_a + k * 16, ps);
+      sts(xx_a + k * 16, xi);
+      sts(px0_a + k * ES, p0);
+    }
+    const int y = bv.yrow(row);
+    if (y >= 0) {
+      int q;
+      const int sd = side_q(j, ny, q);
+      const T* psi = S.psi[1][sd][Q.par_in] + px * (q - 1) + i;
+      const T* x = S.band[1][sd].xi + px * (q - 1) + i;
+      P lo = splat(T(0)), hi = splat(T(0)), xi = splat(T(0));
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+        if (ok >> v & 1u) {
+          lo.v[v] = psi[v];
+          hi.v[v] = psi[px + v];
+          xi.v[v] = x[v];
+        }
+      const int at = (y * cw + c) * 16;
+      sts(ylo_a + at, lo);
+      sts(yhi_a + at, hi);
+      sts(xy_a + at, xi);
     }
   }
-  if (ys >= 0) {
-#pragma unroll
-    for (int f = 0; f <= R; ++f) {
-      P ps;
-#pragma unroll
-      for (int v = 0; v < V; ++v) ps.v[v] = T(0);
-      if (yfc >> f & 1u) {
-        // face f is q of row f - 1 when that row is in the band, else q - 1 of row f
-        const bool up = f > 0 && (yin >> (f - 1) & 1u);
-        int q;
-        const int sd = side_q(1, y0 + r0 + (up ? f - 1 : f), ny, q);
-        const T* psi = S.psi[1][sd][Q.par_in] + px * (up ? q : q - 1);
-#pragma unroll
-        for (int v = 0; v < V; ++v)
-          if (okm >> v & 1u) ps.v[v] = psi[i0 + v];
-      }
-      if (f <= nrow) sts(py_a + f * dyv, ps);
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      P xi;
-#pragma unroll
-      for (int v = 0; v < V; ++v) xi.v[v] = T(0);
-      if (yin >> r & 1u) {
-        int q;
-        const int sd = side_q(1, y0 + r0 + r, ny, q);
-        const T* x = S.band[1][sd].xi + px * (q - 1);
-#pragma unroll
-        for (int v = 0; v < V; ++v)
-          if (okm >> v & 1u) xi.v[v] = x[i0 + v];
-      }
-      if (r < nrow) sts(xy_a + r * dyv, xi);
-    }
-  }
+  const int trow = tl.rows;
+  const bool live = tid < cw * ((h + trow - 1) / trow);
+  const int cv = live ? tid % cw : 0, r0 = live ? tid / cw * trow : 0;  // idle threads shadow the first
+  const int nrow = live ? min(trow, h - r0) : 0;
+  const int i0 = x0 + cv * V;
+  const unsigned okm = ok_of(cv);
+  const bool full = okm == (1u << V) - 1u, fix = !full && nrow > 0;
   P f[R];
 #pragma unroll
   for (int r = 0; r < R; ++r)
@@ -685,12 +692,13 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
   const int cl = __shfl_up_sync(0xffffffffu, base, 1), cr = __shfl_down_sync(0xffffffffu, base, 1);
   const int lds_l = lane == 0 || cl != base - V, lds_r = lane == 31 || cr != base + V;
   // edges: where this thread's go, where the first ring value it fetches is
-  const int64_t slot_words = Q.mail_stride / 2;
+  // (mailbox words as 32-bit numbers)
+  const int slot_words = (int)(Q.mail_stride / 2);
   const int oL = 0, oR = Q.hmax * WPV, oU = 2 * Q.hmax * WPV, oD = (2 * Q.hmax + Q.wmax) * WPV;
   const int nU = tl.nbr[2] >= 0 ? w : 0, nD = tl.nbr[3] >= 0 ? w : 0;
   const int nL = tl.nbr[0] >= 0 ? h : 0, nR = tl.nbr[1] >= 0 ? h : 0;
   const int nring = nU + nD + nL + nR;
-  const unsigned long long* inbox = Q.mail + (int64_t)blockIdx.x * Q.mail_stride;
+  const int inbox = (int)blockIdx.x * (int)Q.mail_stride;
   auto ring = [&](int k, int& cell) -> int {  // ring value k: its cell and mailbox word
     if (k < nU) {
       cell = V + k;
@@ -709,29 +717,89 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
     return oR + k * WPV;
   };
   int ring_cell = 0;
-  const unsigned long long* const ring_at = inbox + (tid < nring ? ring(tid, ring_cell) : 0);
-  const bool top = nU && r0 == 0, bottom = nD && r0 + nrow == h;
-  const bool early = R >= LOOP_EARLY_R && tl.nitem > 0;
-  const bool edge = nrow > 0 && !early &&
-                    (top || bottom || (nL && cv == 0) || (nR && cv == cw - 1));
+  const int ring_at = inbox + (tid < nring ? ring(tid, ring_cell) : 0);
+  const bool early = R >= LOOP_EARLY_R && tl.nedge > 0;
+  // late sends: the mailbox words of this thread's edges, -1 without one
+  const bool send = nring && !early && nrow > 0;
+  const int to_u = send && nU && r0 == 0 ? (int)(tl.nbr[2] * Q.mail_stride) + oD + cv * V * WPV : -1;
+  const int to_d = send && nD && r0 + nrow == h ? (int)(tl.nbr[3] * Q.mail_stride) + oU + cv * V * WPV : -1;
+  const int to_l = send && nL && cv == 0 ? (int)(tl.nbr[0] * Q.mail_stride) + oR + r0 * WPV : -1;
+  const int to_r = send && nR && cv == cw - 1 ? (int)(tl.nbr[1] * Q.mail_stride) + oL + r0 * WPV : -1;
+  const bool edge = to_u >= 0 || to_d >= 0 || to_l >= 0 || to_r >= 0;
   // With several rows per thread the edges are computed first, by all threads
   // (an item each), and sent before the tile's own update, which then hides
-  // their trip (0.8 us when they are sent after it). Items only read the
-  // state; the update computes the same values again. The Dirichlet columns
-  // of an upper or lower row are sent too; nothing reads them.
-  LoopItem im{};
+  // their trip. Items only read the state; the update computes the same values
+  // again. The Dirichlet columns of an upper or lower row are sent too; nothing
+  // reads them.
+  LoopEdge im{};
   int it_base = -1;
-  if (early && tid < tl.nitem) {
-    im = Q.items[tl.item0 + tid];
-    it_base = ((im.rc >> 16) + 1) * pitch + (im.rc & 0xffff) + V;
+  unsigned it_xin = 0;
+  if (early && tid < tl.nedge) {
+    im = Q.edges[tl.edge0 + tid];
+    it_base = ((im.rc >> 16) + 1) * pitch + (im.rc & 0xffff) * V + V;
+    it_xin = xin_of(im.rc & 0xffff);
   }
   const T* __restrict__ fact = S.fact + x0 + px * y0;  // of the tile's first node
   const int ipx = (int)px;
-  const bool fix = !full && nrow > 0;
-  unsigned bm = 0;  // rows with CPML work
+  // The CPML terms of band vector k (row, vector c; centre value cc, its
+  // neighbours read from cur): the damping, and the new state when `put`.
+  auto band_terms = [&](int k, int row, int c, uint32_t at, const P& cc, unsigned ok, unsigned xin,
+                        bool put) -> P {
+    const P fk = get<P>(bf_a + k * 16);
+    P damp = splat(T(0));
+    if (k < nxv) {
+      const T xm = get<T>(at - ES), xp = get<T>(at + V * ES);
+      P ps = get<P>(px_a + k * 16), xo = get<P>(xx_a + k * 16);
+      T p0 = get<T>(px0_a + k * ES);
+      vec_xband(cx_a + c * 16, cxs * ES, cc, xm, xp, fk, xin, ix, ix2, p0, ps, xo, damp);
+      if (put) {
+        sts(px0_a + k * ES, p0);
+        sts(px_a + k * 16, ps);
+        sts(xx_a + k * 16, xo);
+      }
+    }
+    const int y = bv.yrow(row);
+    if (y >= 0) {
+      const P up = get<P>(at - dp), dn = get<P>(at + dp);
+      const int e = (y * cw + c) * 16;
+      P lo = get<P>(ylo_a + e), hi = get<P>(yhi_a + e), xo = get<P>(xy_a + e);
+      vec_psi(lo, splat(cy[row]), splat(cy[cys + row]), vec_sub(cc, up), iy);
+      vec_psi(hi, splat(cy[row + 1]), splat(cy[cys + row + 1]), vec_sub(dn, cc), iy);
+      vec_tail(splat(cy[2 * cys + row]), splat(cy[3 * cys + row]), vec_sub(hi, lo), xo,
+               vec_d2y(up, cc, dn, iy2), fk, iy, damp);
+      if (put) {
+        sts(ylo_a + e, lo);
+        sts(yhi_a + e, hi);
+        sts(xy_a + e, xo);
+      }
+    }
+    if (ok != (1u << V) - 1u) {  // the Dirichlet columns take none
 #pragma unroll
-  for (int r = 0; r < R; ++r)
-    if (r < nrow && (xs >= 0 || ((yfc >> r) & 3u))) bm |= 1u << r;
+      for (int v = 0; v < V; ++v)
+        if (!(ok >> v & 1u)) damp.v[v] = T(0);
+    }
+    return damp;
+  };
+  // The band vectors this thread works on: with one row per thread its own,
+  // inside the update; else numbers tid, tid + nthr, ... after it, spread over
+  // the block (as the owners' own they made the band threads of a full tile
+  // take 8200 cycles where the others took 3200).
+  int bk = -1, brow = 0, bc = 0;
+  unsigned bok = 0, bxin = 0;
+  if (R == 1) {
+    if (nrow > 0) bk = bv.index(r0, cv);
+    brow = r0;
+    bc = cv;
+  } else if (tid < nband) {
+    bk = tid;
+    bv.at(bk, brow, bc);
+  }
+  if (bk >= 0) {
+    bok = ok_of(bc);
+    bxin = xin_of(bc);
+  }
+  const int bcell = (brow + 1) * pitch + bc * V + V;
+  const bool settle = any_src || (nring && !early);
   bool dead = false;  // a wait ran out: no more waiting, the host reports it
   __syncthreads();
 
@@ -743,49 +811,32 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
         rec_to += nrec;
       }
       for (int e = rec_e; e < rec1; e += nthr)
-        S.traces[(Q.it0 + s - 1) * nrec + Q.recs[e].id] =
-            get<T>(cur + Q.recs[e].cell * ES);
+        S.traces[(Q.it0 + s - 1) * nrec + Q.recs[e].id] = get<T>(cur + Q.recs[e].cell * ES);
     }
     const uint32_t tag = Q.tag0 + (uint32_t)s;
-    const int64_t slot = (s & 1) * slot_words;
+    const int slot = (s & 1) * slot_words;
     const bool more = s + 1 < Q.n;
     if (early && more) {
       if (it_base >= 0) {
-        const int row = im.rc >> 16, cc = im.rc & 0xffff;
-        const P fi = ldg_pack<T>(fact + cc + ipx * row);
+        const int row = im.rc >> 16, c = im.rc & 0xffff;
         const uint32_t b = cur + it_base * ES;
-        const P c = get<P>(b), up = get<P>(b - dp), dn = get<P>(b + dp);
+        const P fi = ldg_pack<T>(fact + c * V + ipx * row);
+        const P cc = get<P>(b), up = get<P>(b - dp), dn = get<P>(b + dp);
         const P o = get<P>(nxt + it_base * ES);
         const T xm = get<T>(b - ES), xp = get<T>(b + V * ES);
         P nv, d2x, d2y;
-        vec_update(up, c, dn, o, fi, xm, xp, ix2, iy2, d2x, d2y, nv);
-        if (im.flag & 12) {
-          P damp = splat(T(0));
-          if (im.flag & 4) {
-            const int e = row * nvx + (im.flag >> 16);
-            P ps = get<P>(sb + tl.px + e * 16), xo = get<P>(sb + tl.xx + e * 16);
-            T s0 = get<T>(sb + tl.px0 + e * ES);
-            vec_xband(cx_a + cc * ES, cxs * ES, c, xm, xp, fi, (unsigned)(im.flag >> 8) & ((1u << V) - 1u),
-                      ix, ix2, s0, ps, xo, damp);
-          }
-          if (im.flag & 8) {
-            P lo = get<P>(sb + tl.py + im.py * 16), hi = get<P>(sb + tl.py + (im.py + nyt) * 16);
-            P xo = get<P>(sb + tl.xy + im.xy * 16);
-            vec_psi(lo, splat(cy[row]), splat(cy[cys + row]), vec_sub(c, up), iy);
-            vec_psi(hi, splat(cy[row + 1]), splat(cy[cys + row + 1]), vec_sub(dn, c), iy);
-            vec_tail(splat(cy[2 * cys + row]), splat(cy[3 * cys + row]), vec_sub(hi, lo), xo, d2y, fi,
-                     iy, damp);
-          }
+        vec_update(up, cc, dn, o, fi, xm, xp, ix2, iy2, d2x, d2y, nv);
+        if (im.band >= 0) {
+          const P damp = band_terms(im.band, row, c, b, cc, (1u << V) - 1u, it_xin, false);
 #pragma unroll
           for (int v = 0; v < V; ++v) nv.v[v] += damp.v[v];
         }
-        unsigned long long* m = Q.mail + slot + im.mail;
-        const int one = im.flag & 3;
-        if (one == 0) {
+        unsigned long long* m = Q.mail + (slot + im.mail);
+        if (im.what == 0) {
 #pragma unroll
           for (int v = 0; v < V; ++v) mail_put(m + v * WPV, nv.v[v], tag);
         } else {
-          mail_put(m, one == 1 ? nv.v[0] : nv.v[V - 1], tag);
+          mail_put(m, im.what == 1 ? nv.v[0] : nv.v[V - 1], tag);
         }
       }
       __syncthreads();  // the update below overwrites what the items read
@@ -797,10 +848,10 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
       const uint32_t cb = cur + base * ES, ob = nxt + base * ES;
       P q[R + 2], o[R];
       T xm[R], xp[R];
-      auto neighbours = [&](int r, uint32_t a) {  // of the vector at a, row r
+      auto neighbours = [&](int r, uint32_t a, const P& c) {  // of row r's vector c, at a
         if constexpr (sizeof(T) == 4) {
-          xm[r] = __shfl_up_sync(0xffffffffu, q[r + 1].v[V - 1], 1);
-          xp[r] = __shfl_down_sync(0xffffffffu, q[r + 1].v[0], 1);
+          xm[r] = __shfl_up_sync(0xffffffffu, c.v[V - 1], 1);
+          xp[r] = __shfl_down_sync(0xffffffffu, c.v[0], 1);
           lds_if(a - ES, lds_l, xm[r]);
           lds_if(a + V * ES, lds_r, xp[r]);
         } else {
@@ -812,21 +863,24 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
       lds(cb - dp, q[0]);
       lds(ob, o[0]);
       lds(cb + dp, q[2]);
-      neighbours(0, cb);
+      neighbours(0, cb, q[1]);
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         if (r > 0 && r >= rows) break;
-        if (R >= LOOP_EARLY_R && r == rows - 1 && early && more && tid < nring)
-          ahead = mail_get(ring_at + slot);
         const uint32_t rc = cb + r * dp, ro = ob + r * dp;
         if (r + 1 < R) {
           constexpr int last = R + 1;
           lds(rc + 2 * dp, q[r + 3 < last ? r + 3 : last]);
           lds(ro + dp, o[r + 1 < R ? r + 1 : r]);
-          neighbours(r + 1 < R ? r + 1 : r, rc + dp);
+          neighbours(r + 1 < R ? r + 1 : r, rc + dp, q[r + 2]);
         }
         P nv, d2x, d2y;
         vec_update(q[r], q[r + 1], q[r + 2], o[r], f[r], xm[r], xp[r], ix2, iy2, d2x, d2y, nv);
+        if (R == 1 && bk >= 0) {
+          const P damp = band_terms(bk, brow, bc, rc, q[1], bok, bxin, true);
+#pragma unroll
+          for (int v = 0; v < V; ++v) nv.v[v] += damp.v[v];
+        }
         if (r < nrow) sts(ro, nv);
       }
       if (fix) {  // Dirichlet columns hold 0 (where no source sits)
@@ -835,55 +889,32 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
           for (int v = 0; v < V; ++v)
             if (!(okm >> v & 1u)) sts(ob + r * dp + v * ES, T(0));
       }
+    }
+    if (R >= LOOP_EARLY_R && early && more && tid < nring) ahead = mail_get(Q.mail + (ring_at + slot));
+    if (R > 1 && nband > 0) {
       // CPML: the damping term is added to the stored leapfrog value, as the
       // per-step kernels add it
-      if (bm) {
-        P pyc;  // the new ψ on the face above the row
-        if (yfc & 1u) {
-          const P c = get<P>(cb), up = get<P>(cb - dp);
-          lds(py_a, pyc);
-          vec_psi(pyc, splat(cy[r0]), splat(cy[cys + r0]), vec_sub(c, up), iy);
-          sts(py_a, pyc);
-        }
+      __syncthreads();
+      if (bk >= 0) {
+        const uint32_t at = cur + bcell * ES, to = nxt + bcell * ES;
+        const P cc = get<P>(at);
+        const P damp = band_terms(bk, brow, bc, at, cc, bok, bxin, true);
+        P nv = get<P>(to);
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if (!(bm >> r & 1u)) continue;
-          const uint32_t rc = cb + r * dp, ro = ob + r * dp;
-          const P c = get<P>(rc);
-          P damp = splat(T(0));
-          if (xs >= 0) {
-            const T xm = get<T>(rc - ES), xp = get<T>(rc + V * ES);
-            P ps = get<P>(px_a + r * dxv), xo = get<P>(xx_a + r * dxv);
-            T s0 = get<T>(px0_a + r * dx0);
-            vec_xband(cx_a + cv * 16, cxs * ES, c, xm, xp, f[r], xin, ix, ix2, s0, ps, xo, damp);
-            sts(px0_a + r * dx0, s0);
-            sts(px_a + r * dxv, ps);
-            sts(xx_a + r * dxv, xo);
-          }
-          if ((yfc >> r) & 3u) {
-            const P dn = get<P>(rc + dp);
-            P pyn;
-            if (yfc >> (r + 1) & 1u) {
-              lds(py_a + (r + 1) * dyv, pyn);
-              vec_psi(pyn, splat(cy[r0 + r + 1]), splat(cy[cys + r0 + r + 1]), vec_sub(dn, c), iy);
-              sts(py_a + (r + 1) * dyv, pyn);
-            }
-            if (yin >> r & 1u) {
-              const P up = get<P>(rc - dp);
-              P xo = get<P>(xy_a + r * dyv);
-              vec_tail(splat(cy[2 * cys + r0 + r]), splat(cy[3 * cys + r0 + r]), vec_sub(pyn, pyc), xo,
-                       vec_d2y(up, c, dn, iy2), f[r], iy, damp);
-              sts(xy_a + r * dyv, xo);
-            }
-            pyc = pyn;
-          }
-          P nv = get<P>(ro);
+        for (int v = 0; v < V; ++v) nv.v[v] += damp.v[v];
+        sts(to, nv);
+        for (int k = bk + nthr; k < nband; k += nthr) {
+          const int rc = reinterpret_cast<const int*>(smem + bt_o)[k], row = rc >> 16, c = rc & 0xffff;
+          const int cell = (row + 1) * pitch + c * V + V;
+          const P c2 = get<P>(cur + cell * ES);
+          const P d2 = band_terms(k, row, c, cur + cell * ES, c2, ok_of(c), xin_of(c), true);
+          P n2 = get<P>(nxt + cell * ES);
 #pragma unroll
-          for (int v = 0; v < V; ++v)
-            if (okm >> v & 1u) nv.v[v] += damp.v[v];
-          sts(ro, nv);
+          for (int v = 0; v < V; ++v) n2.v[v] += d2.v[v];
+          sts(nxt + cell * ES, n2);
         }
       }
+      if (settle) __syncthreads();  // owners read their nodes below
     }
     if (any_src) {
       if (one_cell >= 0) {
@@ -919,37 +950,36 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
     if (nring && more) {
       if (edge) {  // this thread's edge nodes to the neighbours' inboxes
         const uint32_t own = nxt + base * ES;
-        unsigned long long* m = Q.mail + slot;
-        if (top) {
-          unsigned long long* q = m + tl.nbr[2] * Q.mail_stride + oD + cv * V * WPV;
+        if (to_u >= 0) {
+          const P e = get<P>(own);
+          unsigned long long* q = Q.mail + (to_u + slot);
 #pragma unroll
-          for (int v = 0; v < V; ++v) mail_put(q + v * WPV, get<T>(own + v * ES), tag);
+          for (int v = 0; v < V; ++v) mail_put(q + v * WPV, e.v[v], tag);
         }
-        if (bottom) {
-          unsigned long long* q = m + tl.nbr[3] * Q.mail_stride + oU + cv * V * WPV;
+        if (to_d >= 0) {
+          const P e = get<P>(own + (nrow - 1) * dp);
+          unsigned long long* q = Q.mail + (to_d + slot);
 #pragma unroll
-          for (int v = 0; v < V; ++v) mail_put(q + v * WPV, get<T>(own + (nrow - 1) * dp + v * ES), tag);
+          for (int v = 0; v < V; ++v) mail_put(q + v * WPV, e.v[v], tag);
         }
-        if (nL && cv == 0) {
-          unsigned long long* q = m + tl.nbr[0] * Q.mail_stride + oR + r0 * WPV;
-          for (int r = 0; r < nrow; ++r) mail_put(q + r * WPV, get<T>(own + r * dp), tag);
-        }
-        if (nR && cv == cw - 1) {
-          unsigned long long* q = m + tl.nbr[1] * Q.mail_stride + oL + r0 * WPV;
-          for (int r = 0; r < nrow; ++r) mail_put(q + r * WPV, get<T>(own + r * dp + (V - 1) * ES), tag);
-        }
+        if (to_l >= 0)
+          for (int r = 0; r < nrow; ++r)
+            mail_put(Q.mail + (to_l + slot + r * WPV), get<T>(own + r * dp), tag);
+        if (to_r >= 0)
+          for (int r = 0; r < nrow; ++r)
+            mail_put(Q.mail + (to_r + slot + r * WPV), get<T>(own + r * dp + (V - 1) * ES), tag);
       }
       // the neighbours' edges into this tile's ring
       if (tid < nring && !dead) {
         T x;
-        if (mail_take(ring_at + slot, tag, x, Q.err, ahead))
+        if (mail_take(Q.mail + (ring_at + slot), tag, x, Q.err, ahead))
           sts(nxt + ring_cell * ES, x);
         else
           dead = true;
         for (int e = tid + nthr; e < nring && !dead; e += nthr) {
           int cell;
           const int word = ring(e, cell);
-          if (mail_take(inbox + slot + word, tag, x, Q.err))
+          if (mail_take(Q.mail + (inbox + slot + word), tag, x, Q.err))
             sts(nxt + cell * ES, x);
           else
             dead = true;
@@ -960,6 +990,7 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
     if (Q.keep) {
       const int64_t it = Q.it0 + s;
       if (it >= Q.keep_first && it < Q.keep_first + Q.keep_count) {
+        if (R > 1 && nband > 0 && !settle) __syncthreads();  // other threads' band terms
         T* g = Q.keep + Q.keep_stride * (it - Q.keep_first) + i0 + px * (y0 + r0);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -991,8 +1022,7 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     if (r >= nrow) break;
-    const int j = y0 + r0 + r;
-    const int64_t g = i0 + px * j;
+    const int64_t g = i0 + px * (y0 + r0 + r);
     const P pc = get<P>(cur + (base + r * pitch) * ES), po = get<P>(nxt + (base + r * pitch) * ES);
     if (full) {
       *reinterpret_cast<P*>(gc + g) = pc;
@@ -1005,35 +1035,43 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
           go[g + v] = po.v[v];
         }
     }
-    if (xs >= 0) {
-      const P ps = get<P>(px_a + r * dxv), xo = get<P>(xx_a + r * dxv);
-      const T p0 = get<T>(px0_a + r * dx0);
+  }
+  for (int k = tid; k < nband; k += nthr) {
+    int row, c;
+    bv.at(k, row, c);
+    const int i = x0 + c * V, j = y0 + row;
+    if (k < nxv) {
+      const unsigned xin = xin_of(c);
+      const P ps = get<P>(px_a + k * 16), xo = get<P>(xx_a + k * 16);
+      const T p0 = get<T>(px0_a + k * ES);
 #pragma unroll
       for (int v = 0; v < V; ++v) {
         if (!(xin >> v & 1u)) continue;
         int q;
-        const int sd = side_q(0, i0 + v, nx, q);
+        const int sd = side_q(i + v, nx, q);
         T* psi = S.psi[0][sd][Q.par_out] + (int64_t)(halo + 1) * j;
         psi[q] = ps.v[v];
-        if (i0 + v == 1 || i0 + v == S.first_r[0])
+        if (i + v == 1 || i + v == S.first_r[0])
           psi[q - 1] = v == 0 ? p0 : ps.v[v == 0 ? 0 : v - 1];
         S.band[0][sd].xi[(int64_t)halo * j + q - 1] = xo.v[v];
       }
     }
-    if (ys >= 0 && (yin >> r & 1u)) {
+    const int y = bv.yrow(row);
+    if (y >= 0) {
+      const unsigned ok = ok_of(c);
       int q;
-      const int sd = side_q(1, j, ny, q);
-      T* psi = S.psi[1][sd][Q.par_out];
-      T* xi = S.band[1][sd].xi + px * (q - 1);
+      const int sd = side_q(j, ny, q);
+      T* psi = S.psi[1][sd][Q.par_out] + i;
+      T* xi = S.band[1][sd].xi + px * (q - 1) + i;
       const bool first = j == 1 || j == S.first_r[1];
-      const P hi = get<P>(py_a + (r + 1) * dyv), lo = get<P>(py_a + r * dyv);
-      const P xo = get<P>(xy_a + r * dyv);
+      const int at = (y * cw + c) * 16;
+      const P lo = get<P>(ylo_a + at), hi = get<P>(yhi_a + at), xo = get<P>(xy_a + at);
 #pragma unroll
       for (int v = 0; v < V; ++v) {
-        if (!(okm >> v & 1u)) continue;
-        psi[px * q + i0 + v] = hi.v[v];
-        if (first) psi[px * (q - 1) + i0 + v] = lo.v[v];
-        xi[i0 + v] = xo.v[v];
+        if (!(ok >> v & 1u)) continue;
+        psi[px * q + v] = hi.v[v];
+        if (first) psi[px * (q - 1) + v] = lo.v[v];
+        xi[v] = xo.v[v];
       }
     }
   }

@@ -91,11 +91,9 @@ class Loop2D {
   std::vector<Shape> shapes_;
   std::vector<Wave> waves_;
   std::vector<LoopTile> tiles_;               // without the shots' lists
-  std::vector<std::vector<int>> owners_;      // per tile: the thread of each vector
   int64_t mail_stride_ = 0;
   int32_t* err_ = nullptr;
-  void* table_ = nullptr;  // threads and edge items
-  size_t o_items_ = 0;
+  void* table_ = nullptr;  // edge items
   void* blob_ = nullptr;  // tiles, shots, entry lists
   size_t blob_bytes_ = 0;
   size_t o_shots_ = 0, o_srcs_ = 0, o_recs_ = 0;
