@@ -191,7 +191,7 @@ __device__ __forceinline__ T adj_g(const AdjStep<T>& A, I o) {
 // stencil lap of G_{t+2} + band, and the gradient accumulation
 // dJ/dF += λ_{t+1} B_t with B_t the Laplacian of p_t (in the working
 // precision) at nodes outside every active band, (p_{t+1} - 2 p_t + p_{t-1})
-// / F (in double) inside one, where adj_sources removes the source term.
+// / F (in double) inside one, where adj_io removes the source term.
 template <typename T, typename I, int ND, bool GRAD>
 __device__ __forceinline__ T adj_update(const AdjStep<T>& A, I o, T l2, T l3, T f, T lap, T band,
                                         bool in_band) {
@@ -272,13 +272,9 @@ __device__ __forceinline__ T adj_shell_node(const AdjStep<T>& A, int i, int j, i
   return adj_update<T, I, ND, GRAD>(A, o, l2, l3, f, lap, band, in_band);
 }
 
-// Nodes of the shell boxes: a box's (x, y) columns numbered row by row,
-// l = (i - x0) + W (j - y0), in runs of 256 per block, one z plane per block;
-// the block's box kind selects the body.
-template <typename T, typename I, bool GRAD>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4) adj_shell(const __grid_constant__ AdjStep<T> A) {
-  // the box of this block: box_blk rises strictly, so a binary search
-  const int blk = blockIdx.x;
+// The box (of A's boxes) of block blk: box_blk rises strictly, so a binary search.
+template <typename T>
+__device__ __forceinline__ int adj_box(const AdjStep<T>& A, int blk) {
   int b = 0, hi = A.nbox - 1;
   while (b < hi) {
     const int mid = (b + hi + 1) >> 1;
@@ -287,6 +283,16 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4) adj_shell(const _
     else
       hi = mid - 1;
   }
+  return b;
+}
+
+// Nodes of the shell boxes in the x bands' zones (and of a generic box): a
+// box's (x, y) columns numbered row by row,
+// l = (i - x0) + W (j - y0), in runs of 256 per block, one z plane per block;
+// the block's box kind selects the body.
+template <typename T, typename I, bool GRAD>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4) adj_shell(const __grid_constant__ AdjStep<T> A) {
+  const int blk = blockIdx.x, b = adj_box(A, blk);
   const Box& B = A.box[b];
   const int W = B.x1 - B.x0 + 1, ncol = W * (B.y1 - B.y0 + 1);
   const int ncb = (ncol + 255) / 256;
@@ -302,16 +308,199 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 4) adj_shell(const _
     adj_shell_node<T, I, 3, GRAD, zx, zy, zz>(A, i, j, k, o, A.lam[o]); \
     break;
   switch (B.kind) {
-    AWC_SHELL(1, 0, 0) AWC_SHELL(2, 0, 0) AWC_SHELL(0, 1, 0) AWC_SHELL(1, 1, 0)
-    AWC_SHELL(2, 1, 0) AWC_SHELL(0, 2, 0) AWC_SHELL(1, 2, 0) AWC_SHELL(2, 2, 0)
-    AWC_SHELL(0, 0, 1) AWC_SHELL(1, 0, 1) AWC_SHELL(2, 0, 1) AWC_SHELL(0, 1, 1)
-    AWC_SHELL(1, 1, 1) AWC_SHELL(2, 1, 1) AWC_SHELL(0, 2, 1) AWC_SHELL(1, 2, 1)
-    AWC_SHELL(2, 2, 1) AWC_SHELL(0, 0, 2) AWC_SHELL(1, 0, 2) AWC_SHELL(2, 0, 2)
-    AWC_SHELL(0, 1, 2) AWC_SHELL(1, 1, 2) AWC_SHELL(2, 1, 2) AWC_SHELL(0, 2, 2)
+    AWC_SHELL(1, 0, 0) AWC_SHELL(2, 0, 0) AWC_SHELL(1, 1, 0) AWC_SHELL(2, 1, 0)
+    AWC_SHELL(1, 2, 0) AWC_SHELL(2, 2, 0) AWC_SHELL(1, 0, 1) AWC_SHELL(2, 0, 1)
+    AWC_SHELL(1, 1, 1) AWC_SHELL(2, 1, 1) AWC_SHELL(1, 2, 1) AWC_SHELL(2, 2, 1)
+    AWC_SHELL(1, 0, 2) AWC_SHELL(2, 0, 2) AWC_SHELL(1, 1, 2) AWC_SHELL(2, 1, 2)
     AWC_SHELL(1, 2, 2) AWC_SHELL(2, 2, 2)
     default: adj_shell_node<T, I, 3, GRAD, 3, 3, 3>(A, i, j, k, o, A.lam[o]);
   }
 #undef AWC_SHELL
+}
+
+// adj_side along y or z (a = 1, 2) for the pair of nodes (i, i + 1) of one row,
+// which have the same entry q: their coefficients are loaded once and their
+// ν and μ, neighbours in memory, as vectors. va, vb: which of the two store.
+template <typename T, typename I>
+__device__ __forceinline__ typename Vec2<T>::type adj_side2(
+    const AdjStep<T>& A, int a, int s, int q, int i, int j, int k, typename Vec2<T>::type gm,
+    typename Vec2<T>::type gc, typename Vec2<T>::type gp, bool va, bool vb) {
+  using V2 = typename Vec2<T>::type;
+  const int h = A.halo;
+  const I step = band_step<I>(A, a);
+  const I nb = band_base<I>(A, a, h, i, j, k), mb = band_base<I>(A, a, h + 1, i, j, k);
+  const V2* __restrict__ nuc = A.nuc[a][s];
+  const T* __restrict__ nu_in = A.nu_in[a][s];
+  auto ld = [](const T* p) { return __ldg(reinterpret_cast<const V2*>(p)); };
+  auto st = [&](T* p, V2 v) {
+    if (va && vb) {
+      *reinterpret_cast<V2*>(p) = v;
+    } else {
+      if (va) p[0] = v.x;
+      if (vb) p[1] = v.y;
+    }
+  };
+  const V2 gv[3] = {gm, gc, gp};
+  V2 w[3], anu[3];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    const int e = q - 2 + m;
+    w[m] = V2{T(0), T(0)};
+    anu[m] = V2{T(0), T(0)};
+    if (e >= 0 && e < h) {
+      const V2 c = __ldg(nuc + e);  // {bK, a}
+      const V2 in = ld(nu_in + nb + (I)e * step);
+      const V2 nu{fma(c.x, in.x, gv[m].x), fma(c.x, in.y, gv[m].y)};
+      anu[m] = V2{mul_rn(c.y, nu.x), mul_rn(c.y, nu.y)};
+      w[m] = V2{fma(c.y, nu.x, gv[m].x), fma(c.y, nu.y, gv[m].y)};
+      if (m == 1) st(A.nu_out[a][s] + nb + (I)e * step, nu);
+    }
+  }
+  const T inv_d = A.inv_d[a];
+  const V2* __restrict__ muc = A.muc[a][s];
+  const T* __restrict__ mu_in = A.mu_in[a][s];
+  T* __restrict__ mu_out = A.mu_out[a][s];
+  V2 f{T(0), T(0)};
+  if (q >= 1) {  // face q - 1
+    const int e = q - 1;
+    const V2 c = __ldg(muc + e);  // {bKh, ah}
+    const V2 in = ld(mu_in + mb + (I)e * step);
+    const V2 mu{fma(c.x, in.x, mul_rn(inv_d, w[0].x - w[1].x)),
+                fma(c.x, in.y, mul_rn(inv_d, w[0].y - w[1].y))};
+    f = V2{mul_rn(c.y, mu.x), mul_rn(c.y, mu.y)};
+    if (q == 1) st(mu_out + mb, mu);
+  }
+  if (q <= h) {  // face q
+    const V2 c = __ldg(muc + q);
+    const V2 in = ld(mu_in + mb + (I)q * step);
+    const V2 mu{fma(c.x, in.x, mul_rn(inv_d, w[1].x - w[2].x)),
+                fma(c.x, in.y, mul_rn(inv_d, w[1].y - w[2].y))};
+    f = V2{f.x - mul_rn(c.y, mu.x), f.y - mul_rn(c.y, mu.y)};
+    if (q >= 1) st(mu_out + mb + (I)q * step, mu);
+  }
+  const T ax = (anu[2].x - T(2) * anu[1].x) + anu[0].x, ay = (anu[2].y - T(2) * anu[1].y) + anu[0].y;
+  return V2{fma(A.inv_d2[a], ax, mul_rn(inv_d, f.x)), fma(A.inv_d2[a], ay, mul_rn(inv_d, f.y))};
+}
+
+// The bracket 1/F (p_{t+1} - 2 p_t + p_{t-1}) of a band node, as adj_update's.
+template <typename T>
+__device__ __forceinline__ double adj_bracket(T f, T pp1, T c, T pm1) {
+  const double fd = (double)f;
+  double r = (double)__frcp_rn((float)fd);
+  r = r * fma(-fd, r, 2.0);
+  r = r * fma(-fd, r, 2.0);
+  return (((double)pp1 - 2.0 * (double)c) + (double)pm1) * r;
+}
+
+// The pair of 3D shell nodes (i, i + 1), i even, outside the x bands' zones, in
+// the zones ZY, ZZ: adj_shell_node for both.
+template <typename T, typename I, bool GRAD, int ZY, int ZZ>
+__device__ __forceinline__ void adj_pair_node(const AdjStep<T>& A, int i, int j, int k, bool va,
+                                              bool vb) {
+  using V2 = typename Vec2<T>::type;
+  const I px = (I)A.px, pl = (I)A.plane;
+  const I o = (I)i + px * (I)j + pl * (I)k;
+  auto ld = [](const T* p) { return __ldg(reinterpret_cast<const V2*>(p)); };
+  auto g2 = [&](I at) {
+    const V2 f = ld(A.F + at), l = ld(A.lam2 + at);
+    return V2{mul_rn(f.x, l.x), mul_rn(f.y, l.y)};
+  };
+  const V2 f = ld(A.F + o), l2 = ld(A.lam2 + o), gc{mul_rn(f.x, l2.x), mul_rn(f.y, l2.y)};
+  const T gl = adj_g(A, o - 1), gr = adj_g(A, o + 2);
+  const V2 ym = g2(o - px), yp = g2(o + px), zm = g2(o - pl), zp = g2(o + pl);
+  V2 lap{second_diff(gl, gc.x, gc.y, A.inv_d2[0]) + second_diff(ym.x, gc.x, yp.x, A.inv_d2[1]),
+         second_diff(gc.x, gc.y, gr, A.inv_d2[0]) + second_diff(ym.y, gc.y, yp.y, A.inv_d2[1])};
+  lap.x += second_diff(zm.x, gc.x, zp.x, A.inv_d2[2]);
+  lap.y += second_diff(zm.y, gc.y, zp.y, A.inv_d2[2]);
+  const int h = A.halo;
+  V2 band{T(0), T(0)};
+  bool in_band = false;
+  if (ZY) {
+    const int q = j - A.off[1][ZY - 1];
+    in_band = q >= 1 && q <= h;
+    const V2 b = adj_side2<T, I>(A, 1, ZY - 1, q, i, j, k, ym, gc, yp, va, vb);
+    band.x += b.x;
+    band.y += b.y;
+  }
+  if (ZZ) {
+    const int q = k - A.off[2][ZZ - 1];
+    in_band = in_band || (q >= 1 && q <= h);
+    const V2 b = adj_side2<T, I>(A, 2, ZZ - 1, q, i, j, k, zm, gc, zp, va, vb);
+    band.x += b.x;
+    band.y += b.y;
+  }
+  const V2 l3 = *reinterpret_cast<const V2*>(A.lam + o);
+  const V2 lam{(T(2) * l2.x - l3.x) + (lap.x + band.x), (T(2) * l2.y - l3.y) + (lap.y + band.y)};
+  if (GRAD) {
+    const T* __restrict__ P = A.p0;
+    const V2 c = ld(P + o);
+    double ba, bb;
+    if (in_band) {
+      const V2 up = ld(A.pp1 + o), dn = ld(A.pm1 + o);
+      ba = adj_bracket(f.x, up.x, c.x, dn.x);
+      bb = adj_bracket(f.y, up.y, c.y, dn.y);
+    } else {
+      const T xl = __ldg(P + o - 1), xr = __ldg(P + o + 2);
+      const V2 y0 = ld(P + o - px), y1 = ld(P + o + px), z0 = ld(P + o - pl), z1 = ld(P + o + pl);
+      T ta = second_diff(xl, c.x, c.y, A.inv_d2[0]) + second_diff(y0.x, c.x, y1.x, A.inv_d2[1]);
+      T tb = second_diff(c.x, c.y, xr, A.inv_d2[0]) + second_diff(y0.y, c.y, y1.y, A.inv_d2[1]);
+      ta += second_diff(z0.x, c.x, z1.x, A.inv_d2[2]);
+      tb += second_diff(z0.y, c.y, z1.y, A.inv_d2[2]);
+      ba = (double)ta;
+      bb = (double)tb;
+    }
+    double2* G = reinterpret_cast<double2*>(A.grad + o);
+    if (va && vb) {
+      double2 g = *G;
+      g.x += (double)lam.x * ba;
+      g.y += (double)lam.y * bb;
+      *G = g;
+    } else {
+      if (va) A.grad[o] += (double)lam.x * ba;
+      if (vb) A.grad[o + 1] += (double)lam.y * bb;
+    }
+  }
+  if (va && vb) {
+    *reinterpret_cast<V2*>(A.lam + o) = lam;
+  } else {
+    if (va) A.lam[o] = lam.x;
+    if (vb) A.lam[o + 1] = lam.y;
+  }
+}
+
+// The shell boxes outside the x bands' zones (kinds with zx = 0), two nodes of
+// a row per thread: half the instructions per node of one node per thread,
+// which bounded the shell (383 thread instructions per node, 41 % of the DRAM
+// rate). 232 x 212 x 232 with halo 20, FP32, alone on the chip: these boxes
+// 45.1 us, the x bands' zones, one node per thread, 51.5 us (their row is a band
+// and its 20 nodes, which pairs do not shorten); all boxes in one kernel of one
+// node per thread 90.8 us. The three kernels run
+// beside each other, the core (51.0 us) among them, so a gradient of 150 steps
+// and two shots gains less: 99.0 to 95.9 ms, 10 us per backward step.
+template <typename T, typename I, bool GRAD>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
+    adj_shell_pair(const __grid_constant__ AdjStep<T> A) {
+  const int b = adj_box(A, (int)blockIdx.x);
+  const Box& B = A.box[b];
+  const int xs = B.x0 & ~1, W = ((B.x1 - xs) >> 1) + 1, ncol = W * (B.y1 - B.y0 + 1);
+  const int ncb = (ncol + 255) / 256;
+  const int r = (int)blockIdx.x - A.box_blk[b];
+  const int kz = A.fastdiv ? (int)(((uint64_t)r * A.box_mncb[b]) >> 32) : r / ncb;
+  const int l = (r - kz * ncb) * 256 + threadIdx.x;
+  if (l >= ncol) return;
+  const int jl = A.fastdiv ? (int)(((uint64_t)l * A.box_mw[b]) >> 32) : l / W;
+  const int i = xs + 2 * (l - jl * W), j = B.y0 + jl, k = B.z0 + kz;
+  const bool va = i >= B.x0, vb = i + 1 <= B.x1;
+  switch (B.kind) {
+    case 3: adj_pair_node<T, I, GRAD, 1, 0>(A, i, j, k, va, vb); break;
+    case 6: adj_pair_node<T, I, GRAD, 2, 0>(A, i, j, k, va, vb); break;
+    case 9: adj_pair_node<T, I, GRAD, 0, 1>(A, i, j, k, va, vb); break;
+    case 12: adj_pair_node<T, I, GRAD, 1, 1>(A, i, j, k, va, vb); break;
+    case 15: adj_pair_node<T, I, GRAD, 2, 1>(A, i, j, k, va, vb); break;
+    case 18: adj_pair_node<T, I, GRAD, 0, 2>(A, i, j, k, va, vb); break;
+    case 21: adj_pair_node<T, I, GRAD, 1, 2>(A, i, j, k, va, vb); break;
+    default: adj_pair_node<T, I, GRAD, 2, 2>(A, i, j, k, va, vb); break;
+  }
 }
 
 // The receiver and source nodes of a 2D step: `flag` marks them (one byte per
@@ -331,7 +520,7 @@ struct AdjIo2 {
 
 // A whole 2D adjoint step in one launch: one thread per interior node, with
 // its receivers' residuals entering λ_{t+3} first and its sources served from
-// its new value (adj_residuals and adj_sources, node by node). A 2D step is a
+// its new value (adj_io, node by node). A 2D step is a
 // few hundred thousand nodes, so what it costs is launches: as four of them on
 // two streams it took 17 us, bound by the host, against 2.4 us in this form
 // (540 x 296, FP32). The launches overlap: the next step's blocks come up while
@@ -593,20 +782,6 @@ __global__ void __launch_bounds__(32 * TY) adj_core_tma(const __grid_constant__ 
   }
 }
 
-// λ_{t+3} -= R_t at the receiver nodes before the step kernels run (the
-// residuals of step t enter λ_{t+1} = R_t + 2 λ_{t+2} - λ_{t+3} + ...), one
-// thread per node, its receivers in receiver order.
-template <typename T>
-__global__ void adj_residuals(T* __restrict__ lam3, const int64_t* __restrict__ node,
-                              const int32_t* __restrict__ off, const int32_t* __restrict__ ids,
-                              int32_t nnode, const T* __restrict__ res_row) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= nnode) return;
-  T v = lam3[node[n]];
-  for (int e = off[n]; e < off[n + 1]; ++e) v -= res_row[ids[e]];
-  lam3[node[n]] = v;
-}
-
 // The residual rows [nt][nrec] in the working precision from a column-major
 // (nt x nrec) double array d: rows[t][r] = traces[t][r] - d[t + nt r] when
 // traces is given (d = observed data), else d itself (the adjoint traces).
@@ -647,15 +822,30 @@ __global__ void __launch_bounds__(256) adj_residual_rows(const T* __restrict__ t
   }
 }
 
-// Per source (one thread, serial over sources for a fixed summation order):
-// the adjoint of the injected value, λ_{t+1} at the source node, and the
-// removal of the source term from the gradient bracket.
+// What a 3D step does besides its nodes, in one launch after it. Block 0: per
+// source (one thread, serial over sources for a fixed summation order) the
+// adjoint of the injected value, λ_{t+1} at the source node, and the removal of
+// the source term from the gradient bracket. The other blocks: λ -= R at the
+// receiver nodes for the step before (the residuals of step t enter
+// λ_{t+1} = R_t + 2 λ_{t+2} - λ_{t+3} + ... as a change of λ_{t+3}), one thread per
+// node, its receivers in receiver order.
 template <typename T>
-__global__ void adj_sources(const T* __restrict__ lamn, const T* __restrict__ F,
-                            const int64_t* __restrict__ node, const int8_t* __restrict__ in_band,
-                            int32_t nsrc, const T* __restrict__ stf_row,
-                            double* __restrict__ grad, T* __restrict__ out_row) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+__global__ void adj_io(const T* __restrict__ lamn, const T* __restrict__ F,
+                       const int64_t* __restrict__ node, const int8_t* __restrict__ in_band,
+                       int32_t nsrc, const T* __restrict__ stf_row, double* __restrict__ grad,
+                       T* __restrict__ out_row, T* __restrict__ lam3,
+                       const int64_t* __restrict__ rnode, const int32_t* __restrict__ off,
+                       const int32_t* __restrict__ ids, int32_t nres,
+                       const T* __restrict__ res_row) {
+  if (blockIdx.x > 0) {
+    const int n = ((int)blockIdx.x - 1) * blockDim.x + threadIdx.x;
+    if (n >= nres) return;
+    T v = lam3[rnode[n]];
+    for (int e = off[n]; e < off[n + 1]; ++e) v -= res_row[ids[e]];
+    lam3[rnode[n]] = v;
+    return;
+  }
+  if (threadIdx.x != 0) return;
   for (int s = 0; s < nsrc; ++s) {
     const int64_t o = node[s];
     if (o < 0) continue;  // rim source: no adjoint
@@ -820,6 +1010,44 @@ Groups group_nodes(const awc_problem* p, int64_t px, const int64_t* pos, int64_t
 // shell is every product of zones but the core's (26 boxes in 3D, 8 in 2D),
 // each with its zone code as kind. When the zones of an axis leave no core
 // node between them, one generic box holds the whole interior.
+// Block ranges of A's boxes, columns of `step` nodes.
+template <typename T>
+void adj_blocks(awc::AdjStep<T>& A, int step) {
+  A.box_blk[0] = 0;
+  A.fastdiv = 1;
+  for (int b = 0; b < A.nbox; ++b) {
+    const awc::Box& B = A.box[b];
+    const int64_t W = step == 2 ? ((B.x1 - (B.x0 & ~1)) >> 1) + 1 : B.x1 - B.x0 + 1;
+    const int64_t ncol = W * (B.y1 - B.y0 + 1);
+    const int64_t ncb = (ncol + 255) / 256, nbz = B.z1 - B.z0 + 1;
+    A.box_blk[b + 1] = (int32_t)(A.box_blk[b] + ncb * nbz);
+    A.box_mw[b] = ((1ull << 32) + (uint64_t)W - 1) / (uint64_t)W;
+    A.box_mncb[b] = ((1ull << 32) + (uint64_t)ncb - 1) / (uint64_t)ncb;
+    // quotients l / W with l < 256 ncb and r / ncb with r < ncb nbz
+    if (256 * ncb * W >= (1ll << 32) || ncb * nbz * ncb >= (1ll << 32)) A.fastdiv = 0;
+  }
+  for (int b = A.nbox; b < 27; ++b) A.box_blk[b + 1] = A.box_blk[b];
+}
+
+// Moves the boxes outside the x bands' zones from A to Z, a copy of A for the
+// pair kernel, and numbers the blocks of both.
+template <typename T>
+void adj_split(awc::AdjStep<T>& A, awc::AdjStep<T>& Z) {
+  Z = A;
+  Z.nbox = 0;
+  int n = 0;
+  for (int b = 0; b < A.nbox; ++b) {
+    const awc::Box B = A.box[b];
+    if (B.kind != awc::ADJ_GENERIC && B.kind % 3 == 0)
+      Z.box[Z.nbox++] = B;
+    else
+      A.box[n++] = B;
+  }
+  A.nbox = n;
+  adj_blocks(A, 1);
+  adj_blocks(Z, 2);
+}
+
 template <typename T>
 void adj_regions(awc::AdjStep<T>& A, int ndim) {
   const int64_t n[3] = {A.nx, A.ny, A.nz}, h = A.halo;
@@ -868,19 +1096,6 @@ void adj_regions(awc::AdjStep<T>& A, int ndim) {
         for (int zx = 0; zx < 3; ++zx)
           if (zx || zy || zz) add(zx, zy, zz, zx + 3 * zy + 9 * zz);
   }
-  A.box_blk[0] = 0;
-  A.fastdiv = 1;
-  for (int b = 0; b < A.nbox; ++b) {
-    const awc::Box& B = A.box[b];
-    const int64_t W = B.x1 - B.x0 + 1, ncol = W * (B.y1 - B.y0 + 1);
-    const int64_t ncb = (ncol + 255) / 256, nbz = B.z1 - B.z0 + 1;
-    A.box_blk[b + 1] = (int32_t)(A.box_blk[b] + ncb * nbz);
-    A.box_mw[b] = ((1ull << 32) + (uint64_t)W - 1) / (uint64_t)W;
-    A.box_mncb[b] = ((1ull << 32) + (uint64_t)ncb - 1) / (uint64_t)ncb;
-    // quotients l / W with l < 256 ncb and r / ncb with r < ncb nbz
-    if (256 * ncb * W >= (1ll << 32) || ncb * nbz * ncb >= (1ll << 32)) A.fastdiv = 0;
-  }
-  for (int b = A.nbox; b < 27; ++b) A.box_blk[b + 1] = A.box_blk[b];
 }
 
 // Offsets fit in int32 when every field (and so every band array) does.
@@ -896,6 +1111,13 @@ void launch_shell(const awc::AdjStep<T>& A, bool grad, bool i64, unsigned blocks
   const auto k = grad ? (i64 ? awc::adj_shell<T, int64_t, true> : awc::adj_shell<T, int32_t, true>)
                       : (i64 ? awc::adj_shell<T, int64_t, false> : awc::adj_shell<T, int32_t, false>);
   k<<<blocks, 256, 0, st>>>(A);
+}
+
+template <typename T>
+void launch_pair(const awc::AdjStep<T>& Z, bool grad, bool i64, unsigned blocks, cudaStream_t st) {
+  const auto k = grad ? (i64 ? awc::adj_shell_pair<T, int64_t, true> : awc::adj_shell_pair<T, int32_t, true>)
+                      : (i64 ? awc::adj_shell_pair<T, int64_t, false> : awc::adj_shell_pair<T, int32_t, false>);
+  k<<<blocks, 256, 0, st>>>(Z);
 }
 
 // One 2D step, as a programmatic dependent of the kernel before it.
@@ -947,14 +1169,12 @@ bool adj_map(CUtensorMap* m, const void* base, const awc::PlanView& V, bool ring
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The adjoint's two streams and five events of the context (created once).
-int adj_streams(awc_ctx* C, cudaStream_t* a, cudaStream_t* b) {
+// The adjoint's streams and events of the context (created once).
+int adj_streams(awc_ctx* C) {
   for (cudaStream_t& s : C->adj_stream)
     if (!s) ADJ_TRY(C, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
   for (cudaEvent_t& e : C->adj_ev)
     if (!e) ADJ_TRY(C, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  *a = C->adj_stream[0];
-  *b = C->adj_stream[1];
   return AWC_OK;
 }
 
@@ -1136,11 +1356,13 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
     }
   }
   adj_regions(A, p->ndim);
+  awc::AdjStep<T> Z{};  // the shell boxes the pair kernel takes
+  adj_split(A, Z);
   const bool has_core = A.core.x0 <= A.core.x1;
   const dim3 core_grid((unsigned)((A.core.x1 - A.core.x0 + 32) / 32),
                        (unsigned)((A.core.y1 - A.core.y0 + 8) / 8),
                        (unsigned)(A.core.z1 - A.core.z0 + 1));
-  const unsigned shell_blocks = (unsigned)A.box_blk[A.nbox];
+  const unsigned shell_blocks = (unsigned)A.box_blk[A.nbox], pair_blocks = (unsigned)Z.box_blk[Z.nbox];
   const bool i64 = NP > (int64_t)INT32_MAX;
   // 3D gradient runs stream the core box through the TMA-fed kernel, in z
   // chunks sized for about four waves of resident blocks
@@ -1273,11 +1495,11 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
       *misfit = J;
     }
   }
-  // backward: the steps run on the adjoint's two streams (core kernel on the
-  // first, shell kernel on the second); segment c - 1 is recomputed on the
+  // backward: the steps run on the adjoint's three streams (the core kernel on
+  // the first, the shell's kernels on the others); segment c - 1 is recomputed on the
   // plan's stream into the other field set meanwhile
-  cudaStream_t bs = nullptr, bs2 = nullptr;
-  if ((rc = adj_streams(C, &bs, &bs2))) return rc;
+  if ((rc = adj_streams(C))) return rc;
+  cudaStream_t bs = C->adj_stream[0], bs2 = C->adj_stream[1], bs3 = C->adj_stream[2];
   cudaEvent_t ev_fork = C->adj_ev[0], ev_join = C->adj_ev[1], ev_rec = C->adj_ev[2];
   cudaEvent_t* ev_free = C->adj_ev + 3;  // set b's backward steps are done
   ADJ_TRY(C, cudaEventRecord(ev_rec, st));  // the set-up above
@@ -1299,6 +1521,7 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
     ADJ_TRY(C, cudaEventRecord(ev_rec, st));
     return AWC_OK;
   };
+  const int32_t nres = (int32_t)RG.node.size();
   int i2 = 0, i3 = 1;  // lam[i2] = λ_{t+2}, lam[i3] = λ_{t+3}
   int par = 0;         // nu[..][par] holds ν_{t+2}
   for (int64_t c = (want_grad ? nseg : 1) - 1; c >= 0; --c) {
@@ -1308,35 +1531,39 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
     for (int64_t t = e - 1; t >= s; --t) {
       // λ_{t+1} overwrites λ_{t+3}, which the step kernels read only at the
       // node they write
-      A.lam2 = lam[i2];
-      A.lam = lam[i3];
-      for (int a = 0; a < p->ndim; ++a)
-        for (int sd = 0; sd < 2; ++sd) {
-          A.nu_in[a][sd] = nu[a][sd][par];
-          A.nu_out[a][sd] = nu[a][sd][par ^ 1];
-          A.mu_in[a][sd] = mu[a][sd][par];
-          A.mu_out[a][sd] = mu[a][sd][par ^ 1];
-        }
-      A.pm1 = want_grad ? seg[b][t - s] : nullptr;
-      A.p0 = want_grad ? seg[b][t - s + 1] : nullptr;
-      A.pp1 = want_grad ? seg[b][t - s + 2] : nullptr;
-      A.grad = grad;
+      for (awc::AdjStep<T>* Y : {&A, &Z}) {
+        Y->lam2 = lam[i2];
+        Y->lam = lam[i3];
+        for (int a = 0; a < p->ndim; ++a)
+          for (int sd = 0; sd < 2; ++sd) {
+            Y->nu_in[a][sd] = nu[a][sd][par];
+            Y->nu_out[a][sd] = nu[a][sd][par ^ 1];
+            Y->mu_in[a][sd] = mu[a][sd][par];
+            Y->mu_out[a][sd] = mu[a][sd][par ^ 1];
+          }
+        Y->pm1 = want_grad ? seg[b][t - s] : nullptr;
+        Y->p0 = want_grad ? seg[b][t - s + 1] : nullptr;
+        Y->pp1 = want_grad ? seg[b][t - s + 2] : nullptr;
+        Y->grad = grad;
+      }
       if (p->ndim == 2) {
         IO.res = res_d + t * nrec;
         IO.stf = stf_d + t * nsrc;
         IO.out = sout_d ? sout_d + t * nsrc : nullptr;
         ADJ_TRY(C, launch_2d(A, IO, want_grad, i64, bs));
       } else {
-        if (!RG.node.empty())
-          awc::adj_residuals<T><<<(unsigned)((RG.node.size() + 127) / 128), 128, 0, bs>>>(
-              A.lam, rnode_d, roff_d, rids_d, (int32_t)RG.node.size(), res_d + t * nrec);
-        const bool fork = has_core && shell_blocks > 0;
+        if (t == nt - 1 && nres > 0)  // later steps: with the sources of the step above
+          awc::adj_io<T><<<1 + (nres + 127) / 128, 128, 0, bs>>>(
+              nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, nullptr, A.lam, rnode_d,
+              roff_d, rids_d, nres, res_d + t * nrec);
+        const bool fork = has_core && shell_blocks + pair_blocks > 0;
         if (fork) {
           ADJ_TRY(C, cudaEventRecord(ev_fork, bs));
           ADJ_TRY(C, cudaStreamWaitEvent(bs2, ev_fork, 0));
+          ADJ_TRY(C, cudaStreamWaitEvent(bs3, ev_fork, 0));
         }
-        if (shell_blocks > 0)
-          launch_shell(A, want_grad, i64, shell_blocks, fork ? bs2 : bs);
+        if (shell_blocks > 0) launch_shell(A, want_grad, i64, shell_blocks, fork ? bs2 : bs);
+        if (pair_blocks > 0) launch_pair(Z, want_grad, i64, pair_blocks, fork ? bs3 : bs);
         if (has_core && use_tma) {
           awc::adj_core_tma<T, ADJ_TY, ADJ_STAGES>
               <<<tma_grid, dim3(32, ADJ_TY), adj_core_smem<T>(), bs>>>(
@@ -1347,11 +1574,16 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
         if (fork) {
           ADJ_TRY(C, cudaEventRecord(ev_join, bs2));
           ADJ_TRY(C, cudaStreamWaitEvent(bs, ev_join, 0));
+          ADJ_TRY(C, cudaEventRecord(C->adj_ev[5], bs3));
+          ADJ_TRY(C, cudaStreamWaitEvent(bs, C->adj_ev[5], 0));
         }
-        if (nsrc > 0)
-          awc::adj_sources<T><<<1, 32, 0, bs>>>(A.lam, A.F, snode_d, sband_d, (int32_t)nsrc,
-                                                stf_d + t * nsrc, grad,
-                                                sout_d ? sout_d + t * nsrc : nullptr);
+        // the sources of this step, and the residuals of the step before it,
+        // which enter what is now λ_{t+2}
+        if (nsrc > 0 || (t > 0 && nres > 0))
+          awc::adj_io<T><<<1 + (t > 0 ? (nres + 127) / 128 : 0), 128, 0, bs>>>(
+              A.lam, A.F, snode_d, sband_d, (int32_t)nsrc, stf_d + t * nsrc, grad,
+              sout_d ? sout_d + t * nsrc : nullptr, lam[i2], rnode_d, roff_d, rids_d, nres,
+              res_d + (t > 0 ? t - 1 : 0) * nrec);
         ADJ_TRY(C, cudaGetLastError());
       }
       std::swap(i2, i3);  // λ_{t+1} is the next step's λ_{t+2}
