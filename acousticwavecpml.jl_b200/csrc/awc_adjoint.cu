@@ -1138,9 +1138,24 @@ cudaError_t launch_2d(const awc::AdjStep<T>& A, const awc::AdjIo2<T>& Q, bool gr
   return cudaLaunchKernelEx(&cfg, k, A, Q);
 }
 
-// Fields of a whole run kept instead of recomputed by segments up to this size
-// (540 x 296, FP32, 600 steps: 0.4 GB).
-constexpr int64_t KEEP_ALL = (int64_t)1 << 30;
+// Whether the gradient keeps every field of the run (one segment: no states
+// saved, nothing recomputed) instead of recomputing segments of `k` steps. Small
+// runs do (KEEP_ALL: 540 x 296, FP32, 600 steps are 0.4 GB), and so do those
+// whose fields take at most 1.5 times what the segments' storage takes (the
+// saved states and two sets of k + 2 fields), up to KEEP_MOST, a sixteenth of
+// the device: memory that buys the recompute, a quarter more steps in the
+// backward pass, beside which the adjoint's kernels slow down. 232 x 212 x 232,
+// FP32, 150 steps by 50, two shots: 95.9 to 79.2 ms
+// (7.1 GB for 5.2 GB). A longer run by the same interval keeps to its segments.
+constexpr int64_t KEEP_ALL = (int64_t)1 << 30, KEEP_MOST = (int64_t)11 << 30;
+bool keep_whole(int64_t nt, int64_t k, int64_t field, int64_t state, int64_t size) {
+  const int64_t nseg = (nt + k - 1) / k;
+  if (nseg < 2) return true;
+  const int64_t whole = (nt + 2) * field * size;
+  if (whole <= KEEP_ALL) return true;
+  const int64_t parts = (nseg * state + 2 * (k + 2) * field) * size;
+  return whole <= KEEP_MOST && whole + state * size <= parts + parts / 2;
+}
 
 // TMA-fed core kernel: tile 64 x 8 nodes, 4 stages.
 constexpr int ADJ_TY = 4, ADJ_STAGES = 4;
@@ -1387,14 +1402,13 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
     A.zchunk = (int32_t)std::max<int64_t>(4, (nzc + chunks - 1) / chunks);
     tma_grid = dim3((unsigned)gx, (unsigned)gy, (unsigned)((nzc + A.zchunk - 1) / A.zchunk));
   }
-  // Checkpoints and segment fields (gradient only). Where one set of all nt
-  // fields takes at most KEEP_ALL bytes (and can be had) the run is one segment:
-  // the forward run keeps every field and nothing is saved or recomputed.
-  const int64_t kask = kchk;
-  if (want_grad && (nt + 2) * fb <= KEEP_ALL) kchk = std::max<int64_t>(kchk, nt);
+  // Checkpoints and segment fields (gradient only)
   int64_t band_elems = 0;
   for (int a = 0; a < p->ndim; ++a) band_elems += 2 * (V.psi_len[a] + V.xi_len[a]);
   const int64_t chk_elems = (3 * NP + band_elems + 63) / 64 * 64;
+  const int64_t kask = kchk;
+  if (want_grad && keep_whole(nt, kask, NP, chk_elems, (int64_t)sizeof(T)))
+    kchk = std::max<int64_t>(kchk, nt);
   int64_t nseg = 0, nfield = 0;
   // segment fields: two sets, so that segment c - 1 is recomputed into one
   // while the backward steps of segment c read the other

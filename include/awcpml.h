@@ -288,8 +288,10 @@ int awc_forward_batch(awc_ctx* ctx, int32_t nmodels, const awc_problem* models,
  * backward pass, the next one beside the current one's adjoint steps
  * (memory: nt / checkpoint_every saved states plus two sets of
  * checkpoint_every + 2 pressure fields, one set when a single segment covers
- * nt). A run whose nt + 2 fields take at most 1 GiB is one segment whatever
- * checkpoint_every: nothing is recomputed, and the result is the same. `traces` (nt x nrec) may be NULL. */
+ * nt). A run whose nt + 2 fields take at most 1 GiB, or at most 1.5 times that
+ * memory and 11 GiB, is one segment whatever checkpoint_every: nothing is
+ * recomputed, and the result is the same (where that memory cannot be had, the
+ * run keeps to checkpoint_every). `traces` (nt x nrec) may be NULL. */
 int awc_misfit_gradient(awc_ctx* ctx, const awc_problem* p, const double* vel,
                         const double* coeffs, const int64_t* possrcs, const double* dt2srctf,
                         const int64_t* posrecs, const double* observed, int32_t checkpoint_every,

@@ -2,7 +2,7 @@
 one launch: dot-product test (FP64, 1e-12 as in test_gpu_adjoint.py) at odd and
 even row lengths, with grids whose x bands' zones leave one node, two nodes or a
 core between them, on sources and receivers that share nodes, repeat, lie in the
-bands and on the Dirichlet rim."""
+bands and on the Dirichlet rim; and segments against runs whose fields are kept."""
 import numpy as np
 import pytest
 
@@ -41,3 +41,23 @@ def test_dot_product(pkg, ctx, n, halo, freetop):
     scale = np.linalg.norm(traces) * np.linalg.norm(r)
     assert abs(lhs) > 1e-6 * scale
     assert abs(lhs - rhs) <= 1e-12 * scale
+
+
+def test_segments_equal_one_segment(pkg, ctx):
+    """100 fields of 12 MB: kept whole for intervals of 100 and 34 steps, by
+    segments for 20; the same bits."""
+    n, nt = (120, 110, 115), 100
+    rng = np.random.default_rng(3)
+    vel = np.asfortranarray(2000.0 + 800.0 * rng.random(n))
+    pos = [[300.0, 400.0, 300.0], [700.0, 20.0, 600.0]]
+    srcs = pkg.Sources(pos[:1], [0.02], [pkg.rickersource1D], 30.0)
+    s = pkg.prepare([(m - 1) * 10.0 for m in n], None, vel, srcs, pkg.Receivers(pos), halo=12,
+                    ppw=1e-9, precision="f64", nt=nt)
+    obs = np.asfortranarray(rng.standard_normal((nt, 2))) * 1e-9
+    want = pkg.adjoint.misfit_gradient(s, obs, nt, ctx)
+    assert np.abs(want[1]).max() > 0.0
+    for every in (34, 20):
+        got = pkg.adjoint.misfit_gradient(s, obs, every, ctx)
+        assert got[0] == want[0]
+        np.testing.assert_array_equal(got[1], want[1])
+        np.testing.assert_array_equal(got[2], want[2])
