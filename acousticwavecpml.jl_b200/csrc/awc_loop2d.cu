@@ -111,11 +111,13 @@ std::vector<int> split(const std::vector<int>& cost, int parts) {
   int64_t total = 0;
   for (int c : cost) total += c;
   std::vector<int> at{0};
-  int64_t have = 0;
+  int64_t have = 0, share = total / parts;
   for (int u = 0; u < n && (int)at.size() < parts; ++u) {
     // the cut nearest to the next equal share
-    const int64_t share = total * (int64_t)at.size() / parts;
-    if (u > at.back() && (have >= share || share - have < have + cost[u] - share)) at.push_back(u);
+    if (u > at.back() && (have >= share || share - have < have + cost[u] - share)) {
+      at.push_back(u);
+      share = total * (int64_t)at.size() / parts;
+    }
     have += cost[u];
   }
   if ((int)at.size() != parts) return {};
@@ -179,6 +181,26 @@ std::vector<Loop2D::Tiling> Loop2D::tilings(const Shape& s, bool f64, int max_ti
     std::fill(ccost.begin(), ccost.end(), 1);
     std::fill(rcost.begin(), rcost.end(), 1);
   }
+  // cuts of the rows into ty parts with the parts' distinct row patterns: the
+  // same for every tx
+  struct Cut {
+    std::vector<int> yb;
+    std::vector<Rows> ys;
+    bool done = false;
+  };
+  std::vector<Cut> cuts(max_tiles + 1);
+  auto cut = [&](int ty) -> const Cut& {
+    Cut& c = cuts[ty];
+    if (c.done) return c;
+    c.done = true;
+    c.yb = split(rcost, ty);
+    for (int t = 0; t < ty && !c.yb.empty(); ++t) {
+      const Rows y = tile_rows(1 + c.yb[t], c.yb[t + 1] - c.yb[t], s.ny, s.halo, s.active[1]);
+      if (std::find(c.ys.begin(), c.ys.end(), y) == c.ys.end()) c.ys.push_back(y);
+    }
+    return c;
+  };
+  std::vector<double> fewer(max_tiles + 1, 1e30);  // lowest cost of fewer tiles so far
   for (int tx = 1; tx <= max_tiles && tx <= cv; ++tx) {
     const std::vector<int> xb = split(ccost, tx);
     // a last tile that starts on the Dirichlet column would send it as its edge
@@ -197,22 +219,22 @@ std::vector<Loop2D::Tiling> Loop2D::tilings(const Shape& s, bool f64, int max_ti
     const int hmax = LOOP_NT / wide * LOOP_ROWS;
     const int ty_lo = (rows + hmax - 1) / hmax, ty_hi = std::min(max_tiles / tx, rows);
     for (int ty = ty_lo; ty <= ty_hi; ++ty) {
-      const std::vector<int> yb = split(rcost, ty);
+      const std::vector<int>& yb = cut(ty).yb;
+      const std::vector<Rows>& ys = cut(ty).ys;
       if (yb.empty()) continue;
-      std::vector<Rows> ys;  // distinct row patterns of the tile rows
-      for (int t = 0; t < ty; ++t) {
-        const Rows y = tile_rows(1 + yb[t], yb[t + 1] - yb[t], s.ny, s.halo, s.active[1]);
-        if (std::find(ys.begin(), ys.end(), y) == ys.end()) ys.push_back(y);
-      }
-      Tiling t;
-      t.tx = tx;
-      t.ty = ty;
-      t.cost = 0.0;
+      const int k = tx * ty;
+      double cost = 0.0;
       bool ok = true;
       for (const auto& c : cols)
         for (const auto& y : ys) {
           if (!ok) break;
           if (thread_rows(c.first, y.all()) == 0) {
+            ok = false;
+            break;
+          }
+          cost = std::max(cost, step_cost(c.first, c.second, y, k > 1));
+          // not better than another tiling of k tiles, or worse than one of fewer
+          if (cost >= best[k].cost || cost > fewer[k]) {
             ok = false;
             break;
           }
@@ -224,14 +246,15 @@ std::vector<Loop2D::Tiling> Loop2D::tilings(const Shape& s, bool f64, int max_ti
           L.ny1 = y.n[2];
           L.nband = band_vectors(c.first, c.second, y);
           ok = (f64 ? tile_smem<double>(L, LOOP_ROWS) : tile_smem<float>(L, LOOP_ROWS)) <= kMaxSmem;
-          t.cost = std::max(t.cost, step_cost(c.first, c.second, y, tx * ty > 1));
         }
-      Tiling& slot = best[tx * ty];
-      if (ok && t.cost < slot.cost) {
-        t.xb = xb;
-        t.yb = yb;
-        slot = std::move(t);
-      }
+      if (!ok) continue;
+      Tiling& t = best[k];
+      t.tx = tx;
+      t.ty = ty;
+      t.xb = xb;
+      t.yb = yb;
+      t.cost = cost;
+      for (int q = k + 1; q <= max_tiles && fewer[q] > cost; ++q) fewer[q] = cost;
     }
   }
   for (int k = 2; k <= max_tiles; ++k)  // at most k tiles
