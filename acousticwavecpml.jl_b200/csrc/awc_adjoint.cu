@@ -528,9 +528,11 @@ struct AdjIo2 {
 template <typename T, typename I, bool GRAD>
 __global__ void __launch_bounds__(256) adj_step2d(const __grid_constant__ AdjStep<T> A,
                                                   const __grid_constant__ AdjIo2<T> Q) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  int i = 1 + (int)(blockIdx.x * 32 + threadIdx.x), j = 1 + (int)(blockIdx.y * 8 + threadIdx.y);
+  // the node goes through the wait, so that no load of its values moves above
+  // it (the compiler takes __ldg for a read of constant memory)
+  asm volatile("griddepcontrol.wait;" : "+r"(i), "+r"(j)::"memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int i = 1 + (int)(blockIdx.x * 32 + threadIdx.x), j = 1 + (int)(blockIdx.y * 8 + threadIdx.y);
   if (i > A.nx - 2 || j > A.ny - 2) return;
   const I o = (I)i + (I)A.px * (I)j;
   T l3 = A.lam[o];
