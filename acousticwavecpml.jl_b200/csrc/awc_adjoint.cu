@@ -1183,7 +1183,7 @@ bool adj_map(CUtensorMap* m, const void* base, const awc::PlanView& V, bool ring
   const cuuint32_t es[3] = {1, 1, 1};
   return enc(m, dt, 3, const_cast<void*>(base), dims, strides, box, es,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+             CU_TENSOR_MAP_L2_PROMOTION_L2_64B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // The adjoint's streams and events of the context (created once).

@@ -939,7 +939,10 @@ int ensure_io(awc_plan* P) {
 // Tensor map of a pitched field of the plan for the core kernel at the
 // current tile height: the pcur box with its ring ((64 + 2A) x (by + 2) x 1,
 // ring = true) or the pold / fact tile (64 x by x 1). Dims (nx, ny, nz),
-// pitched strides.
+// pitched strides. L2 fetches in 64 bytes: a core row starts and ends inside the
+// x bands, whose nodes 256-byte fetches read along, 1 KB rows becoming 1.25 KB
+// (254 MB read per step for 200 MB of nodes at 296 x 276 x 296, FP32: 122.9 us
+// per step with 256, 120.6 with 64; 424 x 404 x 424: 300.7 and 296.9).
 bool field_map(const awc_plan* P, CUtensorMap* m, const void* base, bool ring) {
   PFN_cuTensorMapEncodeTiled_v12000 enc = awc::tensor_map_encoder();
   if (!enc) return false;
@@ -954,7 +957,7 @@ bool field_map(const awc_plan* P, CUtensorMap* m, const void* base, bool ring) {
   const cuuint32_t es[3] = {1, 1, 1};
   return enc(m, dt, 3, const_cast<void*>(base), dims, strides, ring ? box_c : box_i, es,
              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+             CU_TENSOR_MAP_L2_PROMOTION_L2_64B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // Tensor maps of the 3D core kernel: both boxes for each rotating field
@@ -2209,11 +2212,18 @@ int awc_plan_autotune(awc_plan* P, int64_t steps, float* best_ms_per_step) {
   P->depth = 1;
   // phase 1: core tile height and z chunk
   std::vector<std::pair<int32_t, int32_t>> cands;
-  for (int by : {4, 8, 16})
-    for (double waves : {0.5, 1.0, 2.0, 4.0, 8.0}) {
-      const std::pair<int32_t, int32_t> c{by, chunk_for(P, by, waves)};
+  for (int by : {4, 8, 16}) {
+    std::vector<int32_t> chunks;
+    for (double waves : {0.5, 1.0, 2.0, 4.0, 8.0}) chunks.push_back(chunk_for(P, by, waves));
+    // and short chunks whatever the grid: the columns in flight then cover fewer
+    // rows, whose aprons L2 still holds (424 x 404 x 424, FP32: 297 us per step,
+    // 301 with the best chunk of the waves above)
+    if (P->has_core) chunks.push_back(8);
+    for (int32_t zc : chunks) {
+      const std::pair<int32_t, int32_t> c{by, zc};
       if (std::find(cands.begin(), cands.end(), c) == cands.end()) cands.push_back(c);
     }
+  }
   float best = 1e30f;
   std::pair<int32_t, int32_t> win{P->by, P->zchunk};
   for (const auto& c : cands) {
