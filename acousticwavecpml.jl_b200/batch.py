@@ -95,6 +95,11 @@ class Batch:
               self.ctx.handle)
         return a.value, b.value
 
+    def launch_count(self, nsteps=None):
+        """Kernel launches a run of `nsteps` steps (default: all) issues."""
+        n = self.nt if nsteps is None else nsteps
+        return int(_lib.lib().awc_batch_launch_count(self._h, int(n)))
+
     def autotune(self, steps=20):
         ms = ctypes.c_float(0.0)
         check(_lib.lib().awc_batch_autotune(self._h, int(steps), ctypes.byref(ms)),

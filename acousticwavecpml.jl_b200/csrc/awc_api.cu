@@ -3,9 +3,10 @@
 // Responsibilities: argument validation with the reference's error cases
 // (positions inside the model, src/shared/acoustic_3D_xPU.jl:281,289; halo
 // small enough for the band index arithmetic of :12,:68), the FP64 CPML
-// coefficient setup (src/utils.jl:19-57), device buffers, the per-step launch
-// sequence of forward! (:124-167), its capture into CUDA graphs, and the
-// launch-shape autotuner.
+// coefficient setup (src/utils.jl:19-57), device buffers, the launch
+// sequence of forward! (:124-167; 2D runs that fit on the chip are one launch,
+// others one or two per step, captured into CUDA graphs), and the launch-shape
+// autotuner.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>

@@ -1,9 +1,11 @@
 // awc_batch.cu — batched 2D shots over several velocity models.
 //
-// Many shots (sources) over velocity models of uneven size advance together:
-// one kernel launch per time step covers every shot (a persistent grid over
-// the global tile list, awc::step2d_batch), and the nt-step loop is captured
-// once into a CUDA graph. Each shot computes exactly what a single-shot
+// Many shots (sources) over velocity models of uneven size advance together,
+// in one of two ways, the faster one picked by the tuner: through the on-chip
+// loop (awc_loop2d.h), one launch for all the steps of the shots whose tiles
+// fill the SMs together; or one kernel launch per time step for every shot (a
+// persistent grid over the global tile list, awc::step2d_batch), the nt-step
+// loop captured once into a CUDA graph. Each shot computes exactly what a single-shot
 // awc_forward of the same problem computes (the same per-node arithmetic).
 // The reference has no batched API: its solve2D runs one shot per call
 // (src/shared/acoustic_2D_xPU.jl:133-445).
@@ -681,6 +683,13 @@ int awc_batch_get_launch(const awc_batch* B, int32_t* tile_y, int32_t* blocks_pe
   *tile_y = B->ty;
   *blocks_per_sm = B->bps;
   return AWC_OK;
+}
+
+int64_t awc_batch_launch_count(const awc_batch* B, int64_t nsteps) {
+  if (!B || nsteps < 0) return -1;
+  const int64_t n = std::min<int64_t>(nsteps, B->nt - B->step);
+  awc_batch* M = const_cast<awc_batch*>(B);  // the tiling, made on first use
+  return loop_run(M, n) ? M->loop.launches() : n;
 }
 
 int awc_batch_run(awc_batch* B, int64_t nsteps, int32_t use_graph, float* ms) {

@@ -391,7 +391,7 @@ struct Tile3 {
 // shared-memory stages with cp.async.bulk.tensor, each stage with a "full"
 // mbarrier (TMA bytes) and an "empty" mbarrier (one arrival per warp once the
 // warp is done with the stage). Plane k is computed from the stages of planes
-// k-1, k, k+1; loads run up to S-3 planes ahead and warps may drift apart by
+// k-1, k, k+1; loads run up to S-2 planes ahead and warps may drift apart by
 // as much, with no block-wide barrier in the loop. Each thread owns 2 x 2
 // nodes: an x pair read and written as one vector, in two rows, with its
 // values of planes k - 1 and k held in registers.

@@ -7,11 +7,11 @@
 // at 2088 x 1044 in FP32. Here the grid of a shot is cut into tiles, one block
 // per tile and per SM; a block keeps its tile's p_t and p_{t-1} (in place of
 // which p_{t+1} is written) in shared memory, its fact values in registers and
-// the ψ/ξ of its CPML nodes in shared memory, and steps nt times: 2.0, 2.8 and
-// 4.1 us per step on the same grids. What bounds it: on small tiles the edges'
-// trip through L2 (0.8 us), on full ones the issue of the update (1.9 us per
-// 16384 FP32 nodes and SM) and, on the tiles of the CPML bands, the longer
-// dependent chain of a band row.
+// the ψ/ξ of its CPML nodes in shared memory, and steps nt times: 1.8, 2.3 and
+// 4.7 us per step on the same grids. What bounds it: on small tiles the edges'
+// trip through L2 (0.8 us), on full ones the issue of the update (1.7 us per
+// 16384 FP32 nodes and SM) and, on the tiles of the CPML bands, the rounds of
+// band vectors that the block's threads take after it.
 // Only the tile's edge nodes leave the SM: after each step they go to the
 // neighbour tiles' mailboxes in global memory (L2), every 32-bit word of a
 // value paired with the step's tag in one 64-bit store, so the receiver polls

@@ -9,7 +9,8 @@
  * source time functions, position snapping) and hands the arrays to
  * awc_forward(); everything the reference runs through ParallelStencil kernels
  * (update_ψ_*!, update_p!, inject_sources!, record_receivers!, forward!) runs
- * here as one fused CUDA kernel per time step, replayed from a CUDA graph.
+ * here as fused CUDA kernels: a 2D run that fits on the chip as one launch,
+ * others as one (2D) or two (3D) per time step, replayed from a CUDA graph.
  *
  * Conventions shared by every entry point:
  *  - Arrays are host memory, column-major (Julia layout), unless stated.
@@ -155,7 +156,8 @@ void awc_plan_destroy(awc_plan* plan);
 /* Zeroes pressure, ψ, ξ and traces; the next run starts at it = 1. */
 int awc_plan_reset(awc_plan* plan);
 /* Advances `nsteps` time steps (clamped to nt). use_graph = 1 replays a
- * captured CUDA graph, 0 launches the kernels one by one. When ms != NULL the
+ * captured CUDA graph, 0 launches the kernels one by one (a 2D run of 8 steps
+ * or more that fits on the chip is one launch either way). When ms != NULL the
  * device time of the run, measured with CUDA events on the plan's stream, is
  * written there. Returns after the run completes. */
 int awc_plan_run(awc_plan* plan, int64_t nsteps, int32_t use_graph, float* ms);
@@ -180,7 +182,8 @@ int awc_plan_run_snapshots(awc_plan* plan, int64_t nsteps, int64_t nsave, double
 int awc_plan_traces(awc_plan* plan, double* traces);
 int awc_plan_field(awc_plan* plan, double* p);
 /* Number of kernel launches one time step issues (for launch accounting):
- * 2 for a 3D problem with both a core and a CPML band region, else 1. */
+ * 2 for a 3D problem with both a core and a CPML band region, else 1 (of a 2D
+ * run that does not go through the on-chip loop). */
 int32_t awc_plan_launches_per_step(const awc_plan* plan);
 /* Launch shape of a 3D time step, which runs as two kernels over disjoint
  * nodes: the core kernel (nodes outside every CPML band; blocks of 64 x
@@ -213,7 +216,8 @@ int awc_plan_autotune(awc_plan* plan, int64_t steps, float* best_ms_per_step);
 int awc_plan_set_blocking(awc_plan* plan, int32_t depth, int32_t rows, int32_t zchunks);
 int awc_plan_get_blocking(const awc_plan* plan, int32_t* depth, int32_t* rows, int32_t* zchunks);
 /* Kernel launches that a run of nsteps steps from the plan's current step
- * issues (for launch accounting at either depth); -1 on a bad argument. */
+ * issues (for launch accounting at either depth; 1 through the on-chip 2D
+ * loop); -1 on a bad argument. */
 int64_t awc_plan_launch_count(const awc_plan* plan, int64_t nsteps);
 /* Bounded waits of the two-step kernel's TMA pipeline: a wait gives up after
  * `rounds` try-waits of at most round_ns nanoseconds each (default 4096 x
@@ -225,8 +229,11 @@ int awc_plan_set_wait(awc_plan* plan, int32_t rounds, int32_t round_ns, int32_t 
 
 /* ---- Batched 2D shots ----------------------------------------------------
  * Many shots over several 2D velocity models of uneven size advance together:
- * one kernel launch per time step covers every shot, and the nt-step loop is
- * one CUDA graph. Each shot computes what awc_forward computes for the same
+ * through the on-chip 2D loop (one launch for all the steps of the shots whose
+ * tiles fill the SMs together), or with one kernel launch per time step for
+ * every shot, the nt-step loop a CUDA graph. Runs of 8 steps or more of shots
+ * that fit on the chip go through the loop unless awc_batch_autotune finds the
+ * step kernels faster or awc_batch_set_launch asks for them. Each shot computes what awc_forward computes for the same
  * problem. No counterpart in the reference, whose solve2D runs one shot per
  * call (src/shared/acoustic_2D_xPU.jl:133-445). */
 typedef struct awc_shot {
@@ -255,14 +262,19 @@ int64_t awc_batch_step(const awc_batch* batch);
 /* One shot's traces (nt x nrec) and current field (nx*ny), as doubles. */
 int awc_batch_traces(awc_batch* batch, int32_t shot, double* traces);
 int awc_batch_field(awc_batch* batch, int32_t shot, double* p);
-/* Tile height and resident blocks per SM (1..32) of the persistent step
- * kernel; results do not depend on them. tile_y 4, 8 or 16: tiles 64 nodes
+/* Selects the persistent step kernels, with this tile height and these resident
+ * blocks per SM (1..32), in place of the on-chip loop; results do not depend on them. tile_y 4, 8 or 16: tiles 64 nodes
  * wide staged through shared memory by TMA (4 consumer warps of tile_y/4 rows
  * and a producer warp per block); 32 or 64: tiles 32 nodes wide read into
  * registers (4 warps per block, each streaming tile_y/4 rows). */
 int awc_batch_set_launch(awc_batch* batch, int32_t tile_y, int32_t blocks_per_sm);
 int awc_batch_get_launch(const awc_batch* batch, int32_t* tile_y, int32_t* blocks_per_sm);
-/* Times every launch shape on the batch's data, keeps the fastest, resets. */
+/* Kernel launches that a run of nsteps steps from the batch's current step
+ * issues: one per wave of shots through the on-chip loop, one per step with the
+ * step kernels; -1 on a bad argument. */
+int64_t awc_batch_launch_count(const awc_batch* batch, int64_t nsteps);
+/* Times the on-chip loop and every launch shape of the step kernels on the
+ * batch's data, keeps the fastest, resets. */
 int awc_batch_autotune(awc_batch* batch, int64_t steps, float* best_ms_per_step);
 /* create + autotune (nt >= 100) + run(nt) + every shot's traces + destroy;
  * traces[s] is shot s's (nt x nrec) output. */
