@@ -63,6 +63,10 @@ class Shot(ctypes.Structure):
     ]
 
 
+# awc_plan_route
+ROUTE_LOOP, ROUTE_STRIPS, ROUTE_BAND_PAIRS = 1, 2, 4
+
+
 class AwcError(RuntimeError):
     def __init__(self, code, msg):
         super().__init__(f"{_ERRNAMES.get(code, 'error')} ({code}): {msg}")
@@ -115,6 +119,8 @@ SIGNATURES = {
                                              ctypes.POINTER(ctypes.c_int32),
                                              ctypes.POINTER(ctypes.c_int32)]),
     "awc_plan_launch_count": (ctypes.c_int64, [_vp, ctypes.c_int64]),
+    "awc_plan_route": (ctypes.c_int32, [_vp, ctypes.c_int64]),
+    "awc_last_segments": (ctypes.c_int64, [_vp]),
     "awc_forward_decomposed": (ctypes.c_int, [ctypes.POINTER(_vp), ctypes.c_int32, _PP, _vp, _vp,
                                               _vp, _vp, _vp, _vp, _vp]),
     "awc_plan_run_snapshots": (ctypes.c_int, [_vp, ctypes.c_int64, ctypes.c_int64, _vp,

@@ -59,6 +59,10 @@ class Context:
     def last_run_ms(self):
         return float(_lib.lib().awc_last_run_ms(self._h))
 
+    def last_segments(self):
+        """Segments of the last gradient's run (1: all its fields were kept)."""
+        return int(_lib.lib().awc_last_segments(self._h))
+
     @property
     def stream(self):
         """The context's cudaStream_t as an integer handle."""
@@ -180,6 +184,12 @@ class Plan:
         if nsteps is None:
             nsteps = self.problem.nt
         return int(_lib.lib().awc_plan_launch_count(self._h, int(nsteps)))
+
+    def route(self, nsteps=None):
+        """Which kernels a run of nsteps (default: the remaining steps) takes:
+        _lib.ROUTE_LOOP, ROUTE_STRIPS or ROUTE_BAND_PAIRS, else 0."""
+        n = self.problem.nt if nsteps is None else nsteps
+        return int(_lib.lib().awc_plan_route(self._h, int(n)))
 
     def run_snapshots(self, nsteps, nsave, out=None):
         """Advances nsteps and returns the fields after every step whose count

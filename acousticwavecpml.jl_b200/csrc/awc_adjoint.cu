@@ -1426,6 +1426,7 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
     cudaGetLastError();
     kchk = kask;
   }
+  C->segments = nseg;
   std::vector<T*> chk(nseg, nullptr);
   std::vector<T*> seg[2];
   if (want_grad) {

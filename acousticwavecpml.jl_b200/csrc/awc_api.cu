@@ -1873,6 +1873,8 @@ const char* awc_last_error(const awc_ctx* ctx) {
 
 float awc_last_run_ms(const awc_ctx* ctx) { return ctx ? ctx->last_run_ms : 0.f; }
 
+int64_t awc_last_segments(const awc_ctx* ctx) { return ctx ? ctx->segments : -1; }
+
 void* awc_ctx_stream(const awc_ctx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
 
 int awc_ctx_set_autotune(awc_ctx* ctx, int64_t steps) {
@@ -2176,6 +2178,14 @@ int64_t awc_plan_launch_count(const awc_plan* P, int64_t nsteps) {
   // the tile lists (how many launches a pass has) follow the blocking
   if (two_step(P) && ensure_tb(const_cast<awc_plan*>(P)) != AWC_OK) return -1;
   return launch_count(P, std::min<int64_t>(nsteps, P->p.nt - P->step));
+}
+
+int32_t awc_plan_route(const awc_plan* P, int64_t nsteps) {
+  if (!P || nsteps < 0) return -1;
+  if (P->p.ndim == 3) return P->band_wide ? AWC_ROUTE_BAND_PAIRS : 0;
+  const int64_t n = std::min<int64_t>(nsteps, P->p.nt - P->step);
+  if (use_loop(const_cast<awc_plan*>(P), n)) return AWC_ROUTE_LOOP;
+  return strips2d(P) ? AWC_ROUTE_STRIPS : 0;
 }
 
 namespace {

@@ -219,6 +219,14 @@ int awc_plan_get_blocking(const awc_plan* plan, int32_t* depth, int32_t* rows, i
  * issues (for launch accounting at either depth; 1 through the on-chip 2D
  * loop); -1 on a bad argument. */
 int64_t awc_plan_launch_count(const awc_plan* plan, int64_t nsteps);
+/* Which kernels a run of nsteps steps from the plan's current step takes, where
+ * the grid decides: the on-chip 2D loop, 2D steps in vector strips, or node
+ * pairs in the 3D band kernel; 0 for one node per thread, -1 on a bad argument.
+ * Results do not depend on it. */
+#define AWC_ROUTE_LOOP 1
+#define AWC_ROUTE_STRIPS 2
+#define AWC_ROUTE_BAND_PAIRS 4
+int32_t awc_plan_route(const awc_plan* plan, int64_t nsteps);
 /* Bounded waits of the two-step kernel's TMA pipeline: a wait gives up after
  * `rounds` try-waits of at most round_ns nanoseconds each (default 4096 x
  * 1 ms), and the run returns AWC_ERR_TIMEOUT with the context still usable.
@@ -322,6 +330,8 @@ int awc_misfit_gradient_shots(awc_ctx* ctx, const awc_problem* p, int32_t nshot,
                               const double* dt2srctf, const int64_t* posrecs,
                               const double* observed, int32_t checkpoint_every, double* misfit,
                               double* grad_c2);
+/* Segments of the last gradient's run on `ctx` (1: all its fields were kept). */
+int64_t awc_last_segments(const awc_ctx* ctx);
 
 /* The transpose of the linear map from injected source values (dt2srctf,
  * nt x nsrc) to traces (nt x nrec) for fixed c: src_out (nt x nsrc) =
