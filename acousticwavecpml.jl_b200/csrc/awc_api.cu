@@ -810,12 +810,36 @@ void box_blocks(awc_plan* P) {
   for (int b = P->nbox; b < 6; ++b) P->box_blk[b + 1] = P->box_blk[b];
 }
 
-// Bytes of a field from which a 2D step runs in strips (step2d_strip) instead
-// of one node per thread: us per step of the two, FP32 1000 x 1000 7.9 and 7.7,
-// 2000 x 2000 15.4 and 20.5, 5210 x 2604 48 and 89; FP64 2500 x 1500 30 and 42.
+// Whether a 2D step runs in strips (step2d_strip) instead of one node per thread:
+// from STRIP_BYTES a field on (us per step of the two, FP32 1000 x 1000 7.9 and
+// 7.7, 2000 x 2000 20.5 and 15.4, 5210 x 2604 89 and 48; FP64
+// 2500 x 1500 42 and 30), on grids wide enough. A strip's row is 512 bytes, and
+// one that meets an x band takes the time of 2.7 plain ones in FP32 (4 where the
+// band is a few nodes), 2.1 in FP64, so narrow grids lose: 12 M nodes in FP32 with
+// halo 10, one node per thread and strips, 64 columns 107 and 210 us, 256 82 and
+// 99, 384 80 and 78, 640 79 and 61; 6 M in FP64, 66 columns 134 and 140, 130 95
+// and 104, 128 both 77, 256 68 and 56. The costs below are those of a row in plain
+// strips' time per column; they choose the faster of the two to 2 % over 40 to
+// 1500 columns and halos 0 to 18.
 constexpr int64_t STRIP_BYTES = 8000000;
+// The x tiles of w columns, and how many of them meet an active x band.
+void x_tiles(const awc_plan* P, int64_t w, int64_t* tiles, int64_t* band) {
+  const int64_t last = P->p.nx - 2, h = P->p.halo;
+  *tiles = last / w + 1;
+  const int64_t l = P->active[0][0] ? std::min(h, last) / w + 1 : 0;  // [0, l) on the left
+  const int64_t r = P->active[0][1] ? std::max<int64_t>(last + 1 - h, 1) / w : *tiles;  // [r, tiles)
+  *band = l + *tiles - std::max(r, l);
+}
 bool strips2d(const awc_plan* P) {
-  return (P->p.nx - 2) * (P->p.ny - 2) * (int64_t)P->esz >= STRIP_BYTES;
+  if ((P->p.nx - 2) * (P->p.ny - 2) * (int64_t)P->esz < STRIP_BYTES) return false;
+  const bool f32 = P->esz == 4;
+  int64_t strips, sband, tiles, tband;
+  x_tiles(P, 512 / (int64_t)P->esz, &strips, &sband);
+  x_tiles(P, 32, &tiles, &tband);
+  const double per_band = !f32 ? 1.1 : P->p.halo < 8 ? 3.0 : 1.7;
+  const double strip = 512.0 / (double)P->esz * ((double)strips + per_band * (double)sband);
+  const double one = (f32 ? 2.03 : 1.62) * 32.0 * ((double)tiles + (f32 ? 0.4 : 0.6) * (double)tband);
+  return strip < one;
 }
 // Tile of a block of the 2D kernel.
 void tile2d(const awc_plan* P, int64_t* tx, int64_t* ty) {

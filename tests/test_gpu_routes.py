@@ -46,10 +46,14 @@ def test_loop_equals_per_step_kernels_f64(pkg, ctx, grid):
                                             ((3073, 1601, 20, True), "f32"),
                                             ((2690, 1807, 0, False), "f32")])
 def test_strips_equal_batch_kernels(pkg, ctx, grid, precision):
+    _equals_batch(pkg, ctx, grid, precision, pkg._lib.ROUTE_STRIPS)
+
+
+def _equals_batch(pkg, ctx, grid, precision, route):
     s = loop2d._setup(pkg, grid, precision, seed=grid[0])
     p = s["problem"]
     plan = ctx.plan(*_args(s))
-    assert plan.route() == pkg._lib.ROUTE_STRIPS
+    assert plan.route() == route
     plan.run()
     model = pkg.Problem(ndim=2, precision=p.precision, nx=p.nx, ny=p.ny, nz=1, halo=p.halo,
                         freetop=p.freetop, dx=p.dx, dy=p.dy, dz=1.0, dt=p.dt, nt=p.nt, nsrc=0,
@@ -62,6 +66,15 @@ def test_strips_equal_batch_kernels(pkg, ctx, grid, precision):
     np.testing.assert_array_equal(plan.field(), batch.field(0))
     batch.close()
     plan.close()
+
+
+@pytest.mark.parametrize("grid,precision", [((130, 19000, 10, True), "f32"),
+                                            ((260, 9500, 4, True), "f32"),
+                                            ((70, 20000, 18, False), "f64")])
+def test_narrow_grids_take_one_node_per_thread(pkg, ctx, grid, precision):
+    """Beyond the chip, but of few strips a row, most of them in the x bands: strips
+    take up to twice the time there. The same bits as the batch's step kernels."""
+    _equals_batch(pkg, ctx, grid, precision, 0)
 
 
 @pytest.mark.parametrize("precision", ["f64", "f32"])
