@@ -525,10 +525,26 @@ struct AdjIo2 {
 // two streams it took 17 us, bound by the host, against 2.4 us in this form
 // (540 x 296, FP32). The launches overlap: the next step's blocks come up while
 // this one drains (programmatic dependent launch) and wait for its end here.
-template <typename T, typename I, bool GRAD>
-__global__ void __launch_bounds__(256) adj_step2d(const __grid_constant__ AdjStep<T> A,
+// Larger grids are bound by memory: blocks outside the bands take the body
+// without band terms, and OCC blocks fit an SM (8: 32 registers, the band
+// terms spill a few in FP64). us per backward step with its gradient, the band
+// body everywhere with 40 and 48 registers, and this form: 1500 x 800 24.8 and
+// 20.7 in FP32, 35.0 and 30.6 in FP64; 5210 x 2604 331 and 245, 426 and 333.
+// Where one wave of the wider blocks holds the grid (see adj2d_blocks) their
+// registers win: 540 x 296 in FP64 10.2 with 5 blocks, 11.1 with 8.
+template <typename T>
+__host__ __device__ constexpr int adj2d_blocks() { return sizeof(T) == 4 ? 6 : 5; }
+template <typename T, typename I, bool GRAD, int OCC>
+__global__ void __launch_bounds__(256, OCC) adj_step2d(const __grid_constant__ AdjStep<T> A,
                                                   const __grid_constant__ AdjIo2<T> Q) {
-  int i = 1 + (int)(blockIdx.x * 32 + threadIdx.x), j = 1 + (int)(blockIdx.y * 8 + threadIdx.y);
+  const int i0 = 1 + (int)blockIdx.x * 32, j0 = 1 + (int)blockIdx.y * 8;
+  // whether every node of the block lies outside the bands' zones (a band and
+  // the node next to it)
+  const bool core = !(A.active[0][0] && i0 <= A.halo + 1) &&
+                    !(A.active[0][1] && i0 + 31 >= A.nx - A.halo - 2) &&
+                    !(A.active[1][0] && j0 <= A.halo + 1) &&
+                    !(A.active[1][1] && j0 + 7 >= A.ny - A.halo - 2);
+  int i = i0 + (int)threadIdx.x, j = j0 + (int)threadIdx.y;
   // the node goes through the wait, so that no load of its values moves above
   // it (the compiler takes __ldg for a read of constant memory)
   asm volatile("griddepcontrol.wait;" : "+r"(i), "+r"(j)::"memory");
@@ -549,7 +565,8 @@ __global__ void __launch_bounds__(256) adj_step2d(const __grid_constant__ AdjSte
     g = lo;
     for (int e = Q.roff[g]; e < Q.roff[g + 1]; ++e) l3 -= Q.res[Q.rids[e]];
   }
-  const T lam = adj_shell_node<T, I, 2, GRAD, 3, 3, 0>(A, i, j, 0, o, l3);
+  const T lam = core ? adj_shell_node<T, I, 2, GRAD, 0, 0, 0>(A, i, j, 0, o, l3)
+                     : adj_shell_node<T, I, 2, GRAD, 3, 3, 0>(A, i, j, 0, o, l3);
   if (g >= 0)
     for (int e = Q.soff[g]; e < Q.soff[g + 1]; ++e) {
       const int s = Q.sids[e];
@@ -1125,11 +1142,18 @@ void launch_pair(const awc::AdjStep<T>& Z, bool grad, bool i64, unsigned blocks,
 // One 2D step, as a programmatic dependent of the kernel before it.
 template <typename T>
 cudaError_t launch_2d(const awc::AdjStep<T>& A, const awc::AdjIo2<T>& Q, bool grad, bool i64,
-                      cudaStream_t st) {
-  const auto k = grad ? (i64 ? awc::adj_step2d<T, int64_t, true> : awc::adj_step2d<T, int32_t, true>)
-                      : (i64 ? awc::adj_step2d<T, int64_t, false> : awc::adj_step2d<T, int32_t, false>);
+                      int num_sms, cudaStream_t st) {
+  constexpr int FEW = awc::adj2d_blocks<T>();
+  const dim3 grid((unsigned)((A.nx - 2 + 31) / 32), (unsigned)((A.ny - 2 + 7) / 8));
+  const bool one_wave = (int64_t)grid.x * grid.y <= (int64_t)FEW * num_sms;
+  const auto k = grad ? (i64        ? awc::adj_step2d<T, int64_t, true, 8>
+                         : one_wave ? awc::adj_step2d<T, int32_t, true, FEW>
+                                    : awc::adj_step2d<T, int32_t, true, 8>)
+                      : (i64        ? awc::adj_step2d<T, int64_t, false, 8>
+                         : one_wave ? awc::adj_step2d<T, int32_t, false, FEW>
+                                    : awc::adj_step2d<T, int32_t, false, 8>);
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)((A.nx - 2 + 31) / 32), (unsigned)((A.ny - 2 + 7) / 8));
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(32, 8);
   cfg.stream = st;
   cudaLaunchAttribute at[1];
@@ -1567,7 +1591,7 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
         IO.res = res_d + t * nrec;
         IO.stf = stf_d + t * nsrc;
         IO.out = sout_d ? sout_d + t * nsrc : nullptr;
-        ADJ_TRY(C, launch_2d(A, IO, want_grad, i64, bs));
+        ADJ_TRY(C, launch_2d(A, IO, want_grad, i64, C->num_sms, bs));
       } else {
         if (t == nt - 1 && nres > 0)  // later steps: with the sources of the step above
           awc::adj_io<T><<<1 + (nres + 127) / 128, 128, 0, bs>>>(
