@@ -838,7 +838,7 @@ bool strips2d(const awc_plan* P) {
   x_tiles(P, 32, &tiles, &tband);
   const double per_band = !f32 ? 1.1 : P->p.halo < 8 ? 3.0 : 1.7;
   const double strip = 512.0 / (double)P->esz * ((double)strips + per_band * (double)sband);
-  const double one = (f32 ? 2.03 : 1.62) * 32.0 * ((double)tiles + (f32 ? 0.4 : 0.6) * (double)tband);
+  const double one = (f32 ? 2.03 : 1.6) * 32.0 * ((double)tiles + (f32 ? 0.4 : 0.6) * (double)tband);
   return strip < one;
 }
 // Tile of a block of the 2D kernel.
