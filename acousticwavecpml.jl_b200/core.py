@@ -73,6 +73,11 @@ class Context:
         runs for each new 3D problem shape (0 disables it)."""
         check(_lib.lib().awc_ctx_set_autotune(self._h, int(steps)), self._h)
 
+    def set_keep_limit(self, nbytes=-1):
+        """The most bytes by which a gradient may exceed the memory its
+        checkpoint_every asks for (0: never; -1: the library's rule)."""
+        check(_lib.lib().awc_ctx_set_keep_limit(self._h, int(nbytes)), self._h)
+
     def forward(self, problem, vel, coeffs, possrcs, dt2srctf, posrecs, traces, pfinal=None):
         """awc_forward on host buffers (numpy arrays or pinned torch tensors)."""
         rc = _lib.lib().awc_forward(self._h, ctypes.byref(problem), _ptr(vel), _ptr(coeffs),

@@ -925,7 +925,16 @@ struct DevMem {
   size_t next = 0;
   void* sum = nullptr;  // the multi-shot gradient sum, outside the per-call blocks
   size_t sum_bytes = 0;
+  size_t refused = SIZE_MAX;  // the smallest arena of whole runs that was not to be had
   void begin() { next = 0; }
+  // Whether the next block is held in this size, and what asking for another
+  // size gives back.
+  bool holds(size_t bytes) const { return next < blocks.size() && blocks[next].second == bytes; }
+  size_t rest() const {
+    size_t n = 0;
+    for (size_t k = next; k < blocks.size(); ++k) n += blocks[k].second;
+    return n;
+  }
   void release() {
     for (auto& b : blocks) cudaFree(b.first);
     blocks.clear();
@@ -933,6 +942,7 @@ struct DevMem {
     if (sum) cudaFree(sum);
     sum = nullptr;
     sum_bytes = 0;
+    refused = SIZE_MAX;
   }
   cudaError_t get_sum(double** out, size_t bytes) {
     if (sum_bytes != bytes) {
@@ -1164,23 +1174,41 @@ cudaError_t launch_2d(const awc::AdjStep<T>& A, const awc::AdjIo2<T>& Q, bool gr
   return cudaLaunchKernelEx(&cfg, k, A, Q);
 }
 
+// Bytes of the saved states and the segments' fields for segments of k steps.
+int64_t arena_bytes(int64_t nt, int64_t k, int64_t field, int64_t state, int64_t size) {
+  const int64_t nseg = (nt + k - 1) / k;
+  return (nseg * state + (nseg > 1 ? 2 : 1) * (std::min(k, nt) + 2) * field) * size;
+}
+
 // Whether the gradient keeps every field of the run (one segment: no states
 // saved, nothing recomputed) instead of recomputing segments of `k` steps. Small
 // runs do (KEEP_ALL: 540 x 296, FP32, 600 steps are 0.4 GB), and so do those
-// whose fields take at most 1.5 times what the segments' storage takes (the
-// saved states and two sets of k + 2 fields), up to KEEP_MOST, a sixteenth of
-// the device: memory that buys the recompute, a quarter more steps in the
+// whose arena is at most 1.5 times the segments', up to a sixteenth of the
+// device: memory that buys the recompute, a quarter more steps in the
 // backward pass, beside which the adjoint's kernels slow down. 232 x 212 x 232,
-// FP32, 150 steps by 50, two shots: 95.9 to 79.2 ms
-// (7.1 GB for 5.2 GB). A longer run by the same interval keeps to its segments.
-constexpr int64_t KEEP_ALL = (int64_t)1 << 30, KEEP_MOST = (int64_t)11 << 30;
-bool keep_whole(int64_t nt, int64_t k, int64_t field, int64_t state, int64_t size) {
-  const int64_t nseg = (nt + k - 1) / k;
-  if (nseg < 2) return true;
-  const int64_t whole = (nt + 2) * field * size;
-  if (whole <= KEEP_ALL) return true;
-  const int64_t parts = (nseg * state + 2 * (k + 2) * field) * size;
-  return whole <= KEEP_MOST && whole + state * size <= parts + parts / 2;
+// FP32, 150 steps by 50, two shots: 95.9 to 79.2 ms (7.1 GB for 5.2 GB). A longer
+// run by the same interval keeps to its segments (from about 180 steps on there).
+// `limit` (awc_ctx_set_keep_limit): the most bytes beyond the segments' arena, or
+// negative. A sixteenth of the device stays free beside an arena that is not held
+// yet, and what could not be had is not asked for again.
+constexpr int64_t KEEP_ALL = (int64_t)1 << 30;
+bool keep_whole(const DevMem& mem, int64_t nt, int64_t k, int64_t field, int64_t state,
+                int64_t size, int64_t limit) {
+  const int64_t whole = arena_bytes(nt, nt, field, state, size);
+  const int64_t parts = arena_bytes(nt, k, field, state, size);
+  if (whole <= parts) return true;
+  if (limit >= 0 && whole - parts > limit) return false;
+  const int64_t fields = (nt + 2) * field * size;
+  if (fields > KEEP_ALL && 2 * whole > 3 * parts) return false;
+  if (mem.holds((size_t)whole)) return true;
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const int64_t room = (int64_t)total / 16;
+  return (fields <= KEEP_ALL || fields <= room) && (size_t)whole < mem.refused &&
+         whole + room <= (int64_t)(free + mem.rest());
 }
 
 // TMA-fed core kernel: tile 64 x 8 nodes, 4 stages.
@@ -1428,28 +1456,33 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
     A.zchunk = (int32_t)std::max<int64_t>(4, (nzc + chunks - 1) / chunks);
     tma_grid = dim3((unsigned)gx, (unsigned)gy, (unsigned)((nzc + A.zchunk - 1) / A.zchunk));
   }
+  // what the outputs need, ahead of the arena below, which takes what it can get
+  const int64_t N = p->nx * p->ny * V.nz;
+  double *dense = nullptr, *sd = nullptr;
+  if (grad_out) ADJ_TRY(C, mem.get(&dense, N * sizeof(double)));
+  if (src_out && nsrc > 0) ADJ_TRY(C, mem.get(&sd, nt * nsrc * sizeof(double)));
   // Checkpoints and segment fields (gradient only)
   int64_t band_elems = 0;
   for (int a = 0; a < p->ndim; ++a) band_elems += 2 * (V.psi_len[a] + V.xi_len[a]);
   const int64_t chk_elems = (3 * NP + band_elems + 63) / 64 * 64;
   const int64_t kask = kchk;
-  if (want_grad && keep_whole(nt, kask, NP, chk_elems, (int64_t)sizeof(T)))
+  if (want_grad && nt > 0 && keep_whole(mem, nt, kask, NP, chk_elems, (int64_t)sizeof(T), C->keep_limit))
     kchk = std::max<int64_t>(kchk, nt);
-  int64_t nseg = 0, nfield = 0;
-  // segment fields: two sets, so that segment c - 1 is recomputed into one
-  // while the backward steps of segment c read the other
-  int nset = 1;
   T* arena = nullptr;  // one allocation for the saved states and the segments' fields
   while (want_grad) {
-    nseg = (nt + kchk - 1) / kchk;
-    nset = nseg > 1 ? 2 : 1;
-    nfield = std::min<int64_t>(kchk, nt) + 2;
-    const cudaError_t e = mem.get(&arena, (nseg * chk_elems + nset * nfield * NP) * sizeof(T));
+    const int64_t bytes = arena_bytes(nt, kchk, NP, chk_elems, (int64_t)sizeof(T));
+    const cudaError_t e = mem.get(&arena, (size_t)bytes);
     if (e == cudaSuccess) break;
     if (kchk == kask) ADJ_TRY(C, e);
     cudaGetLastError();
+    mem.refused = std::min<size_t>(mem.refused, (size_t)bytes);
     kchk = kask;
   }
+  // segment fields: two sets, so that segment c - 1 is recomputed into one
+  // while the backward steps of segment c read the other
+  const int64_t nseg = want_grad ? (nt + kchk - 1) / kchk : 0;
+  const int64_t nfield = std::min<int64_t>(kchk, nt) + 2;
+  const int nset = nseg > 1 ? 2 : 1;
   C->segments = nseg;
   std::vector<T*> chk(nseg, nullptr);
   std::vector<T*> seg[2];
@@ -1638,23 +1671,18 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
   ADJ_TRY(C, cudaStreamWaitEvent(st, ev_join, 0));
   // outputs
   if (want_grad) {
-    const int64_t N = p->nx * p->ny * V.nz;
     const int blocks = (int)std::min<int64_t>((N + 255) / 256, (int64_t)C->num_sms * 16);
     if (grad_sum) {
       awc::scale_unpitch_add<<<blocks, 256, 0, st>>>(grad, grad_sum, N, p->nx, V.px,
                                                      p->dt * p->dt);
       ADJ_TRY(C, cudaGetLastError());
     } else {
-      double* dense;
-      ADJ_TRY(C, mem.get(&dense, N * sizeof(double)));
       awc::scale_unpitch<<<blocks, 256, 0, st>>>(grad, dense, N, p->nx, V.px, p->dt * p->dt);
       ADJ_TRY(C, cudaGetLastError());
       ADJ_TRY(C, awc::copy_to_host(C, grad_out, dense, N * sizeof(double), st));
     }
   }
   if (src_out && nsrc > 0) {
-    double* sd;
-    ADJ_TRY(C, mem.get(&sd, nt * nsrc * sizeof(double)));
     awc::to_double<T><<<(unsigned)std::min<int64_t>((nt * nsrc + 255) / 256, 4096), 256, 0, st>>>(
         sout_d, sd, nt * nsrc);
     ADJ_TRY(C, cudaGetLastError());

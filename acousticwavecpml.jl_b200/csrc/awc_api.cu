@@ -1908,6 +1908,12 @@ int awc_ctx_set_autotune(awc_ctx* ctx, int64_t steps) {
   return AWC_OK;
 }
 
+int awc_ctx_set_keep_limit(awc_ctx* ctx, int64_t bytes) {
+  if (!ctx) return set_err(nullptr, AWC_ERR_INVALID, "ctx is NULL");
+  ctx->keep_limit = std::max<int64_t>(bytes, -1);
+  return AWC_OK;
+}
+
 int awc_plan_create(awc_ctx* ctx, const awc_problem* p, const double* vel, const double* coeffs,
                     const int64_t* possrcs, const double* dt2srctf, const int64_t* posrecs,
                     awc_plan** out) {
@@ -1922,13 +1928,16 @@ int awc_plan_create(awc_ctx* ctx, const awc_problem* p, const double* vel, const
     if (!vel || !coeffs) return set_err(&ctx->err, AWC_ERR_INVALID, "vel/coeffs are NULL");
     Lifted L;
     lift_1d(p, vel, coeffs, possrcs, posrecs, &L);
-    if ((rc = forward_impl(ctx, &L.p, L.vel.data(), L.coeffs.data(), L.possrcs.data(), dt2srctf,
-                           L.posrecs.data(), out, true)))
-      return rc;
+    rc = awc::with_room(ctx, [&] {
+      return forward_impl(ctx, &L.p, L.vel.data(), L.coeffs.data(), L.possrcs.data(), dt2srctf,
+                          L.posrecs.data(), out, true);
+    });
+    if (rc) return rc;
     (*out)->is1d = true;
     return AWC_OK;
   }
-  return forward_impl(ctx, p, vel, coeffs, possrcs, dt2srctf, posrecs, out);
+  return awc::with_room(
+      ctx, [&] { return forward_impl(ctx, p, vel, coeffs, possrcs, dt2srctf, posrecs, out); });
 }
 
 void awc_plan_destroy(awc_plan* plan) {
@@ -2370,7 +2379,10 @@ int forward_cached(awc_ctx* ctx, const awc_problem* p, const double* vel, const 
       return rc;
     }
   } else {
-    if ((rc = forward_impl(ctx, p, vel, coeffs, possrcs, dt2srctf, posrecs, &P, lifted1d))) return rc;
+    rc = awc::with_room(ctx, [&] {
+      return forward_impl(ctx, p, vel, coeffs, possrcs, dt2srctf, posrecs, &P, lifted1d);
+    });
+    if (rc) return rc;
     P->is1d = lifted1d;
     // a new 3D shape: pick its launch shape once, on its own data
     if (p->ndim == 3 && ctx->autotune_steps > 0 && p->nt >= 100 &&

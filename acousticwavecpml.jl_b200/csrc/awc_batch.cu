@@ -526,6 +526,11 @@ int awc_batch_create(awc_ctx* C, int32_t nmodels, const awc_problem* models,
   B->staging_len = staging;
   B->arena_bytes = off;
   cudaError_t e = cudaMalloc((void**)&B->arena, off);
+  if (e == cudaErrorMemoryAllocation && C->adj_mem) {
+    cudaGetLastError();
+    C->adj_release();  // the adjoint's memory, held between its calls
+    e = cudaMalloc((void**)&B->arena, off);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     delete B;

@@ -30,6 +30,7 @@ struct awc_ctx {
   awc_plan* adj_plan = nullptr;
   void* adj_mem = nullptr;
   std::function<void()> adj_release;
+  int64_t keep_limit = -1;  // awc_ctx_set_keep_limit
   // the adjoint's backward steps run on their own three streams, so that a
   // segment's recompute (on `stream`) overlaps the previous segment's
   // backward steps; events: fork, join, recomputed, segment set 0/1 free, the
@@ -95,6 +96,18 @@ cudaError_t copy_to_host(awc_ctx* C, void* dst, const void* src, size_t bytes, c
 // Sets the calling thread's last error (awc_last_error(NULL)) and, when ctx
 // is not NULL, the context's; returns code.
 int fail(awc_ctx* ctx, int code, const char* msg);
+
+// Runs make(), which creates a plan or a batch, and once more after giving back
+// the adjoint's memory where the device had no room beside it.
+template <typename F>
+int with_room(awc_ctx* C, F make) {
+  int rc = make();
+  if (rc == AWC_ERR_OOM && C->adj_mem) {
+    C->adj_release();
+    rc = make();
+  }
+  return rc;
+}
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
 // dependency on libcuda); NULL when the driver does not offer it.

@@ -299,7 +299,8 @@ int awc_forward_batch(awc_ctx* ctx, int32_t nmodels, const awc_problem* models,
  * checkpoint_every + 2 pressure fields of a segment and the adjoint fields)
  * stay allocated in the context between calls of one shape, so that a
  * sequence of gradients of one survey allocates once; a call of another
- * shape replaces them and awc_destroy frees them.
+ * shape replaces them, a plan or batch that the device has no room for beside
+ * them frees them, and so does awc_destroy.
  *
  * awc_misfit_gradient: J = 1/2 Σ_t Σ_r (traces[t,r] - observed[t,r])² of the
  * shot described like awc_forward, and dJ/d(c²) per node (nx*ny[*nz],
@@ -308,10 +309,11 @@ int awc_forward_batch(awc_ctx* ctx, int32_t nmodels, const awc_problem* models,
  * backward pass, the next one beside the current one's adjoint steps
  * (memory: nt / checkpoint_every saved states plus two sets of
  * checkpoint_every + 2 pressure fields, one set when a single segment covers
- * nt). A run whose nt + 2 fields take at most 1 GiB, or at most 1.5 times that
- * memory and 11 GiB, is one segment whatever checkpoint_every: nothing is
- * recomputed, and the result is the same (where that memory cannot be had, the
- * run keeps to checkpoint_every). `traces` (nt x nrec) may be NULL. */
+ * nt). A run whose nt + 2 fields take at most 1 GiB, or with its first state at
+ * most 1.5 times that memory and a sixteenth of the device, is one segment
+ * whatever checkpoint_every: nothing is recomputed, and the result is the same. The run
+ * keeps to checkpoint_every where less than a sixteenth of the device would
+ * stay free, or where awc_ctx_set_keep_limit says so. `traces` (nt x nrec) may be NULL. */
 int awc_misfit_gradient(awc_ctx* ctx, const awc_problem* p, const double* vel,
                         const double* coeffs, const int64_t* possrcs, const double* dt2srctf,
                         const int64_t* posrecs, const double* observed, int32_t checkpoint_every,
@@ -330,6 +332,10 @@ int awc_misfit_gradient_shots(awc_ctx* ctx, const awc_problem* p, int32_t nshot,
                               const double* dt2srctf, const int64_t* posrecs,
                               const double* observed, int32_t checkpoint_every, double* misfit,
                               double* grad_c2);
+/* The most bytes by which a gradient's saved states and fields may exceed what
+ * checkpoint_every asks for, for the sake of one segment: 0 holds every run to
+ * checkpoint_every, -1 (the default) leaves it to the rule above. */
+int awc_ctx_set_keep_limit(awc_ctx* ctx, int64_t bytes);
 /* Segments of the last gradient's run on `ctx` (1: all its fields were kept). */
 int64_t awc_last_segments(const awc_ctx* ctx);
 
