@@ -2392,9 +2392,13 @@ int forward_cached(awc_ctx* ctx, const awc_problem* p, const double* vel, const 
     }
   }
   ctx->cache.push_back(P);
-  while (ctx->cache.size() > 2) {
-    delete ctx->cache.front();
-    ctx->cache.erase(ctx->cache.begin());
+  // the two most recent shapes of 1D lines and of 2D and 3D grids each: a line's
+  // plan is small, and a grid's (an autotuned one in 3D) does not make way for it
+  auto kind = [&](const awc_plan* q) { return q->is1d == lifted1d; };
+  if (std::count_if(ctx->cache.begin(), ctx->cache.end(), kind) > 2) {
+    const auto old = std::find_if(ctx->cache.begin(), ctx->cache.end(), kind);
+    delete *old;
+    ctx->cache.erase(old);
   }
   if ((rc = awc_plan_run(P, p->nt, 1, &ctx->last_run_ms))) return rc;
   if (traces && (rc = awc_plan_traces(P, traces))) return rc;
