@@ -145,6 +145,7 @@ SIGNATURES = {
     "awc_batch_traces": (ctypes.c_int, [_vp, ctypes.c_int32, _vp]),
     "awc_batch_field": (ctypes.c_int, [_vp, ctypes.c_int32, _vp]),
     "awc_batch_set_launch": (ctypes.c_int, [_vp, ctypes.c_int32, ctypes.c_int32]),
+    "awc_batch_set_wait": (ctypes.c_int, [_vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32]),
     "awc_batch_launch_count": (ctypes.c_int64, [_vp, ctypes.c_int64]),
     "awc_batch_get_launch": (ctypes.c_int, [_vp, ctypes.POINTER(ctypes.c_int32),
                                             ctypes.POINTER(ctypes.c_int32)]),

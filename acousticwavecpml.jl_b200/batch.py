@@ -89,6 +89,11 @@ class Batch:
         check(_lib.lib().awc_batch_set_launch(self._h, int(tile_y), int(blocks_per_sm)),
               self.ctx.handle)
 
+    def set_wait(self, rounds=4096, round_ns=1000000, withhold=-1):
+        """Plan.set_wait for the batch's runs through the on-chip loop."""
+        check(_lib.lib().awc_batch_set_wait(self._h, int(rounds), int(round_ns), int(withhold)),
+              self.ctx.handle)
+
     def get_launch(self):
         a, b = ctypes.c_int32(), ctypes.c_int32()
         check(_lib.lib().awc_batch_get_launch(self._h, ctypes.byref(a), ctypes.byref(b)),

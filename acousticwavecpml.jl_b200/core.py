@@ -215,8 +215,9 @@ class Plan:
         return [np.asfortranarray(out[j].T) for j in range(got.value)]
 
     def set_wait(self, rounds=4096, round_ns=1000000, withhold=-1):
-        """Bounded-wait budget of the two-step kernel's pipeline; `withhold`
-        (tests of the timeout path only) makes every block skip one load."""
+        """Bounded-wait budget of the two-step kernel's pipeline and of the
+        on-chip 2D loop's edges; `withhold` (tests of the timeout path only)
+        makes every block skip one load, or one tile send no edges."""
         check(_lib.lib().awc_plan_set_wait(self._h, int(rounds), int(round_ns), int(withhold)),
               self.ctx.handle)
 

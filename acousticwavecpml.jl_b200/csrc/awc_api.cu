@@ -1431,6 +1431,8 @@ int loop_range(awc_plan* P, int64_t start, int64_t n, StepState& stt, cudaStream
   for (int64_t m = 0; m < n % 6; ++m) stt.step1();
   for (int b = 0; b < 3; ++b) sp.out[b] = stt.ord[b];
   sp.par_out = stt.psi_par;
+  sp.wait.ns = (unsigned long long)P->wait_rounds * (unsigned long long)P->wait_ns;
+  sp.wait.withhold = P->withhold;
   if (P->keep && P->keep_count > 0) {
     sp.keep = P->keep[0];
     sp.keep_stride = P->keep_count > 1

@@ -75,6 +75,7 @@ struct awc_batch {
   // a launch shape of the per-step kernels was chosen
   awc::Loop2D loop;
   bool use_loop = true, loop_ready = false;
+  awc::LoopWait wait;
   std::vector<std::vector<int32_t>> h_rec_off, h_rec_ids;  // receiver groups per shot
   double* staging = nullptr;  // inside the arena (read-out)
   int64_t staging_len = 0;
@@ -441,6 +442,7 @@ int launch_batch_loop(awc_batch* B, int64_t start, int64_t n, cudaStream_t st) {
   }
   sp.par_in = (int32_t)(start & 1);
   sp.par_out = (int32_t)((start + n) & 1);
+  sp.wait = B->wait;
   return B->loop.run(B->ctx, sp, st);
 }
 
@@ -680,6 +682,16 @@ int awc_batch_set_launch(awc_batch* B, int32_t tile_y, int32_t blocks_per_sm) {
   B->ty = tile_y;
   B->bps = blocks_per_sm;
   B->use_loop = false;
+  return AWC_OK;
+}
+
+int awc_batch_set_wait(awc_batch* B, int32_t rounds, int32_t round_ns, int32_t withhold) {
+  if (!B) return awc::fail(nullptr, AWC_ERR_INVALID, "batch is NULL");
+  if (rounds < 1 || round_ns < 1 || round_ns > 10000000 || withhold < -1)
+    return awc::fail(B->ctx, AWC_ERR_INVALID,
+                     "rounds >= 1, round_ns in [1, 1e7] and withhold >= -1 are required");
+  B->wait.ns = (unsigned long long)rounds * (unsigned long long)round_ns;
+  B->wait.withhold = withhold;
   return AWC_OK;
 }
 

@@ -611,6 +611,8 @@ int Loop2D::launch(awc_ctx* C, const LoopSpan& span, cudaStream_t st) {
     Q.keep_first = span.keep_first;
     Q.keep_count = span.keep_count;
     Q.err = err_;
+    Q.wait_ns = span.wait.ns;
+    Q.withhold = span.wait.withhold;
     tag_ += (uint32_t)span.n;
     const void* k = loop_kernel<T>(wv.R);
     LOOP_TRY(C, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));

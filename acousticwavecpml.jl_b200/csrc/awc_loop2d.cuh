@@ -21,8 +21,10 @@
 // edges of step t + 1, which that neighbour sent after reading step t.
 //
 // The blocks wait for one another, so a launch is cooperative (every block
-// resident). Every wait is bounded (about 4 s): on a timeout the kernel sets
-// *err and all blocks leave.
+// resident). Every wait is bounded (LoopRun::wait_ns): a thread whose wait runs
+// out sets *err and waits no more, nor does any thread that sees *err set while it
+// waits; the blocks then run to the end on the edges they have, and the host
+// reports the run as failed.
 //
 // Every node is computed with the functions the per-step kernels use
 // (awc_kernels.cuh), on the same operands in the same order, so results are
@@ -121,6 +123,8 @@ struct LoopRun {
   T* keep;
   int64_t keep_stride, keep_first, keep_count;
   int32_t* err;
+  unsigned long long wait_ns;  // limit of a wait for an edge value
+  int32_t withhold;            // tests only: the tile that sends no edges, or -1
 };
 
 // The units (vector columns or rows) of a tile that hold nodes of an axis's
@@ -271,10 +275,11 @@ __device__ __forceinline__ unsigned long long mail_get(const unsigned long long*
   return w;
 }
 // Bounded wait for the word of `tag` at q (w: an earlier read of it, or 0, a tag
-// that is never used): about 4 s, or until another
+// that is never used): `limit` ns, or until another
 // thread of the launch has raised *err. False when it gives up.
 __device__ __forceinline__ bool mail_wait(const unsigned long long* q, uint32_t tag,
-                                          unsigned long long& w, const int32_t* err) {
+                                          unsigned long long& w, const int32_t* err,
+                                          unsigned long long limit) {
   unsigned long long t0 = 0;
   for (uint32_t spin = 0;; ++spin) {
     if ((uint32_t)(w >> 32) == tag) return true;  // w: 0 or what an earlier read gave
@@ -283,20 +288,22 @@ __device__ __forceinline__ bool mail_wait(const unsigned long long* q, uint32_t 
       unsigned long long t;
       asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
       if (t0 == 0) t0 = t;
-      if (t - t0 > 4000000000ull || *(volatile const int32_t*)err) return false;
+      if (t - t0 > limit || *(volatile const int32_t*)err) return false;
     }
   }
 }
 __device__ __forceinline__ bool mail_take(const unsigned long long* q, uint32_t tag, float& x,
-                                          const int32_t* err, unsigned long long w = 0) {
-  if (!mail_wait(q, tag, w, err)) return false;
+                                          const int32_t* err, unsigned long long limit,
+                                          unsigned long long w = 0) {
+  if (!mail_wait(q, tag, w, err, limit)) return false;
   x = __uint_as_float((uint32_t)w);
   return true;
 }
 __device__ __forceinline__ bool mail_take(const unsigned long long* q, uint32_t tag, double& x,
-                                          const int32_t* err, unsigned long long lo = 0) {
+                                          const int32_t* err, unsigned long long limit,
+                                          unsigned long long lo = 0) {
   unsigned long long hi = 0;
-  if (!mail_wait(q, tag, lo, err) || !mail_wait(q + 1, tag, hi, err)) return false;
+  if (!mail_wait(q, tag, lo, err, limit) || !mail_wait(q + 1, tag, hi, err, limit)) return false;
   x = __longlong_as_double((long long)((lo & 0xffffffffull) | (hi << 32)));
   return true;
 }
@@ -719,8 +726,9 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
   int ring_cell = 0;
   const int ring_at = inbox + (tid < nring ? ring(tid, ring_cell) : 0);
   const bool early = R >= LOOP_EARLY_R && tl.nedge > 0;
+  const bool mute = (int)blockIdx.x == Q.withhold;
   // late sends: the mailbox words of this thread's edges, -1 without one
-  const bool send = nring && !early && nrow > 0;
+  const bool send = nring && !early && nrow > 0 && !mute;
   const int to_u = send && nU && r0 == 0 ? (int)(tl.nbr[2] * Q.mail_stride) + oD + cv * V * WPV : -1;
   const int to_d = send && nD && r0 + nrow == h ? (int)(tl.nbr[3] * Q.mail_stride) + oU + cv * V * WPV : -1;
   const int to_l = send && nL && cv == 0 ? (int)(tl.nbr[0] * Q.mail_stride) + oR + r0 * WPV : -1;
@@ -734,7 +742,7 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
   LoopEdge im{};
   int it_base = -1;
   unsigned it_xin = 0;
-  if (early && tid < tl.nedge) {
+  if (early && tid < tl.nedge && !mute) {
     im = Q.edges[tl.edge0 + tid];
     it_base = ((im.rc >> 16) + 1) * pitch + (im.rc & 0xffff) * V + V;
     it_xin = xin_of(im.rc & 0xffff);
@@ -972,14 +980,14 @@ __global__ void __launch_bounds__(LOOP_NT, 1) loop2d(const __grid_constant__ Loo
       // the neighbours' edges into this tile's ring
       if (tid < nring && !dead) {
         T x;
-        if (mail_take(Q.mail + (ring_at + slot), tag, x, Q.err, ahead))
+        if (mail_take(Q.mail + (ring_at + slot), tag, x, Q.err, Q.wait_ns, ahead))
           sts(nxt + ring_cell * ES, x);
         else
           dead = true;
         for (int e = tid + nthr; e < nring && !dead; e += nthr) {
           int cell;
           const int word = ring(e, cell);
-          if (mail_take(Q.mail + (inbox + slot + word), tag, x, Q.err))
+          if (mail_take(Q.mail + (inbox + slot + word), tag, x, Q.err, Q.wait_ns))
             sts(nxt + cell * ES, x);
           else
             dead = true;

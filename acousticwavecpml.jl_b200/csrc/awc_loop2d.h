@@ -35,6 +35,13 @@ struct LoopShotHost {
   const std::vector<int32_t>* rec_ids = nullptr;
 };
 
+// Limit of a wait for an edge value, and the tile of each launch that sends no
+// edges (tests of the timeout; -1: none).
+struct LoopWait {
+  unsigned long long ns = 4096000000ull;
+  int32_t withhold = -1;
+};
+
 // Where the state of the first and last step lives (buffer numbers of p_t,
 // p_{t-1} and the third field; ψ parity), and the fields to keep (see
 // LoopRun).
@@ -43,6 +50,7 @@ struct LoopSpan {
   int32_t in[3] = {}, out[3] = {}, par_in = 0, par_out = 0;
   void* keep = nullptr;
   int64_t keep_stride = 0, keep_first = 0, keep_count = 0;
+  LoopWait wait;
 };
 
 // A set of shots that run through the loop: one launch per wave of shots

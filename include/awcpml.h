@@ -232,7 +232,9 @@ int32_t awc_plan_route(const awc_plan* plan, int64_t nsteps);
  * 1 ms), and the run returns AWC_ERR_TIMEOUT with the context still usable.
  * withhold >= 0 exists to test that path: the producer of every block skips
  * the plane load with that index, so that its consumers' wait runs out;
- * -1 (the default) loads every plane. */
+ * -1 (the default) loads every plane. A wait of the on-chip 2D loop for an edge
+ * value gives up after rounds x round_ns in all; there the tile with the number
+ * `withhold` sends no edges. */
 int awc_plan_set_wait(awc_plan* plan, int32_t rounds, int32_t round_ns, int32_t withhold);
 
 /* ---- Batched 2D shots ----------------------------------------------------
@@ -276,6 +278,8 @@ int awc_batch_field(awc_batch* batch, int32_t shot, double* p);
  * and a producer warp per block); 32 or 64: tiles 32 nodes wide read into
  * registers (4 warps per block, each streaming tile_y/4 rows). */
 int awc_batch_set_launch(awc_batch* batch, int32_t tile_y, int32_t blocks_per_sm);
+/* awc_plan_set_wait for the batch's runs through the on-chip loop. */
+int awc_batch_set_wait(awc_batch* batch, int32_t rounds, int32_t round_ns, int32_t withhold);
 int awc_batch_get_launch(const awc_batch* batch, int32_t* tile_y, int32_t* blocks_per_sm);
 /* Kernel launches that a run of nsteps steps from the batch's current step
  * issues: one per wave of shots through the on-chip loop, one per step with the
