@@ -422,14 +422,17 @@ bool loop_run(awc_batch* B, int64_t n) {
          (B->loop_ready || B->loop.fits(B->ctx, B->prec == AWC_F64, loop_shots(B)));
 }
 
+// The loop's tables (once).
+int prepare_loop(awc_batch* B) {
+  if (B->loop_ready) return AWC_OK;
+  const int rc = B->loop.prepare(B->ctx, B->prec == AWC_F64, loop_shots(B), (int32_t*)(B->arena + B->err));
+  B->loop_ready = rc == AWC_OK;
+  return rc;
+}
+
 // n steps of every shot from `start`: each wave of shots advances all n steps
 // in one launch before the next wave starts.
 int launch_batch_loop(awc_batch* B, int64_t start, int64_t n, cudaStream_t st) {
-  if (!B->loop_ready) {
-    const int rc = B->loop.prepare(B->ctx, B->prec == AWC_F64, loop_shots(B), (int32_t*)(B->arena + B->err));
-    if (rc) return rc;
-    B->loop_ready = true;
-  }
   awc::LoopSpan sp;
   sp.it0 = start;
   sp.n = n;
@@ -720,7 +723,7 @@ int awc_batch_run(awc_batch* B, int64_t nsteps, int32_t use_graph, float* ms) {
   int rc;
   const bool loop = loop_run(B, n);  // a launch per wave: nothing to capture
   if (loop) use_graph = 0;
-  if (!loop && (rc = ensure_layout(B))) return rc;
+  if ((rc = loop ? prepare_loop(B) : ensure_layout(B))) return rc;
   cudaGraphExec_t ex = nullptr;
   if (use_graph) {
     const uint64_t key = (uint64_t)B->ty | ((uint64_t)B->bps << 8);

@@ -429,6 +429,8 @@ int Loop2D::lay_out(awc_ctx* C) {
       for (int r = 0; L.nbr[1] >= 0 && r < L.h; ++r) item(r, cw - 1, L.nbr[1], oL + r * WPV, 2);
     }
   }
+  for (const Wave& wv : waves_)
+    LOOP_TRY(C, cudaFuncSetAttribute(loop_kernel<T>(wv.R), cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
   const size_t eb = edges.size() * sizeof(LoopEdge);
   if (table_) cudaFree(table_);
   table_ = nullptr;
@@ -615,7 +617,6 @@ int Loop2D::launch(awc_ctx* C, const LoopSpan& span, cudaStream_t st) {
     Q.withhold = span.wait.withhold;
     tag_ += (uint32_t)span.n;
     const void* k = loop_kernel<T>(wv.R);
-    LOOP_TRY(C, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
     void* args[] = {&Q};
     LOOP_TRY(C, cudaLaunchCooperativeKernel(k, dim3((unsigned)wv.ntiles), dim3((unsigned)wv.threads),
                                             args, (size_t)wv.smem, st));
