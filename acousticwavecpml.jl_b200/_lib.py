@@ -120,6 +120,7 @@ SIGNATURES = {
                                              ctypes.POINTER(ctypes.c_int32)]),
     "awc_plan_launch_count": (ctypes.c_int64, [_vp, ctypes.c_int64]),
     "awc_plan_route": (ctypes.c_int32, [_vp, ctypes.c_int64]),
+    "awc_ctx_set_loop_blocks": (ctypes.c_int, [_vp, ctypes.c_int32]),
     "awc_ctx_set_keep_limit": (ctypes.c_int, [_vp, ctypes.c_int64]),
     "awc_last_segments": (ctypes.c_int64, [_vp]),
     "awc_forward_decomposed": (ctypes.c_int, [ctypes.POINTER(_vp), ctypes.c_int32, _PP, _vp, _vp,

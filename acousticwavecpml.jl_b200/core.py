@@ -73,6 +73,11 @@ class Context:
         runs for each new 3D problem shape (0 disables it)."""
         check(_lib.lib().awc_ctx_set_autotune(self._h, int(steps)), self._h)
 
+    def set_loop_blocks(self, blocks=-1):
+        """Most blocks of an on-chip 2D loop's launch (0: no loop; -1: one per SM
+        of the device)."""
+        check(_lib.lib().awc_ctx_set_loop_blocks(self._h, int(blocks)), self._h)
+
     def set_keep_limit(self, nbytes=-1):
         """The most bytes by which a gradient may exceed the memory its
         checkpoint_every asks for (0: never; -1: the library's rule)."""

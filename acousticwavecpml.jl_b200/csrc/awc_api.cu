@@ -309,6 +309,7 @@ struct awc_plan {
   // 2D: the on-chip time loop (awc_loop2d.cuh), when the grid fits it
   awc::Loop2D loop;
   int32_t loop_fits = -1;    // -1 not looked at since the model was uploaded
+  int32_t loop_blocks = 0;   // the context's at that time
   bool loop_ready = false;   // its lists match the current shot
   std::vector<int32_t> h_rec_off, h_rec_ids;  // receiver groups (host copy)
   // run state
@@ -1411,8 +1412,11 @@ awc::LoopShotHost loop_shot(const awc_plan* P) {
 // it, for long enough, its kept fields (if any) evenly spaced in memory.
 bool use_loop(awc_plan* P, int64_t n) {
   if (P->p.ndim != 2 || n < awc::kLoopMinSteps) return false;
-  if (P->loop_fits < 0)
+  if (P->loop_fits < 0 || P->loop_blocks != P->ctx->loop_blocks) {
+    P->loop_blocks = P->ctx->loop_blocks;
+    P->loop_ready = false;
     P->loop_fits = P->loop.fits(P->ctx, P->p.precision == AWC_F64, {loop_shot(P)}) ? 1 : 0;
+  }
   if (!P->loop_fits) return false;
   for (int64_t m = 2; m < P->keep_count; ++m)
     if ((char*)P->keep[m] - (char*)P->keep[m - 1] != (char*)P->keep[1] - (char*)P->keep[0])
@@ -1420,8 +1424,10 @@ bool use_loop(awc_plan* P, int64_t n) {
   return true;
 }
 
-// n steps from `start` in one launch; stt becomes the state after them.
-int loop_range(awc_plan* P, int64_t start, int64_t n, StepState& stt, cudaStream_t st) {
+// n steps from `start` in one launch; stt becomes the state after them. Where the
+// launch is refused (awc::kLoopRefused) nothing ran and stt is as it was.
+int loop_range(awc_plan* P, int64_t start, int64_t n, StepState& state, cudaStream_t st) {
+  StepState stt = state;
   awc::LoopSpan sp;
   sp.it0 = start;
   sp.n = n;
@@ -1441,7 +1447,10 @@ int loop_range(awc_plan* P, int64_t start, int64_t n, StepState& stt, cudaStream
     sp.keep_first = P->keep_first;
     sp.keep_count = P->keep_count;
   }
-  return P->loop.run(P->ctx, sp, st);
+  const int rc = P->loop.run(P->ctx, sp, st);
+  if (rc == awc::kLoopRefused) P->loop_fits = 0;
+  if (rc == AWC_OK) state = stt;
+  return rc;
 }
 
 // Launches steps [start, start + n) from state `stt` (updated to the state
@@ -1492,10 +1501,10 @@ int prepare_launch(awc_plan* P, bool loop = false) {
   int rc;
   if (loop) {
     if (P->loop_ready) return AWC_OK;
-    if ((rc = P->loop.prepare(P->ctx, P->p.precision == AWC_F64, {loop_shot(P)}, P->err_flag)))
-      return rc;
-    P->loop_ready = true;
-    return AWC_OK;
+    rc = P->loop.prepare(P->ctx, P->p.precision == AWC_F64, {loop_shot(P)}, P->err_flag);
+    P->loop_ready = rc == AWC_OK;
+    if (rc == AWC_ERR_OOM) P->loop_fits = 0;  // the caller goes step by step
+    return rc;
   }
   if ((rc = ensure_io(P))) return rc;
   if (P->p.ndim == 3 && P->has_core && (rc = ensure_maps(P))) return rc;
@@ -1853,6 +1862,7 @@ int awc_create(awc_ctx** out, int32_t device) {
   awc_ctx* C = new awc_ctx();
   C->device = device;
   C->num_sms = prop.multiProcessorCount;
+  C->loop_blocks = C->num_sms;
   if (cudaStreamCreateWithFlags(&C->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&C->stream2, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&C->ev0) != cudaSuccess || cudaEventCreate(&C->ev1) != cudaSuccess ||
@@ -1907,6 +1917,14 @@ int awc_ctx_set_autotune(awc_ctx* ctx, int64_t steps) {
   if (!ctx) return set_err(nullptr, AWC_ERR_INVALID, "ctx is NULL");
   if (steps < 0) return set_err(&ctx->err, AWC_ERR_INVALID, "steps must be >= 0");
   ctx->autotune_steps = steps;
+  return AWC_OK;
+}
+
+int awc_ctx_set_loop_blocks(awc_ctx* ctx, int32_t blocks) {
+  if (!ctx) return set_err(nullptr, AWC_ERR_INVALID, "ctx is NULL");
+  if (blocks < -1 || blocks > 4096)
+    return set_err(&ctx->err, AWC_ERR_INVALID, "blocks must be -1 or in [0, 4096]");
+  ctx->loop_blocks = blocks < 0 ? ctx->num_sms : blocks;
   return AWC_OK;
 }
 
@@ -1984,10 +2002,15 @@ int awc_plan_run(awc_plan* P, int64_t nsteps, int32_t use_graph, float* ms) {
   if (ms) *ms = 0.f;
   if (n <= 0) return AWC_OK;
   int rc;
-  const bool loop = use_loop(P, n);  // one launch: nothing to capture
-  if (loop) use_graph = 0;
-  if ((rc = prepare_launch(P, loop))) return rc;
+  bool loop = use_loop(P, n);
+  if (loop && (rc = prepare_launch(P, true))) {
+    if (rc != AWC_ERR_OOM) return rc;
+    loop = false;
+  }
+  if (!loop && (rc = prepare_launch(P))) return rc;
   cudaGraphExec_t ex = nullptr;
+  const int32_t graph = use_graph;
+  if (loop) use_graph = 0;  // one launch: nothing to capture
   if (use_graph && (rc = get_graph(P, P->step, n, &ex))) return rc;
   CUDA_TRY(&C->err, cudaEventRecord(C->ev0, C->stream));
   if (use_graph) {
@@ -1995,7 +2018,9 @@ int awc_plan_run(awc_plan* P, int64_t nsteps, int32_t use_graph, float* ms) {
   }
   StepState end = P->state;
   if (loop) {
-    if ((rc = loop_range(P, P->step, n, end, C->stream))) return rc;
+    rc = loop_range(P, P->step, n, end, C->stream);
+    if (rc == awc::kLoopRefused) return awc_plan_run(P, nsteps, graph, ms);  // step by step
+    if (rc) return rc;
   } else if (!use_graph) {
     if ((rc = launch_range(P, P->step, n, end, C->stream))) return rc;
   } else {
@@ -2037,8 +2062,12 @@ int awc_plan_run_snapshots(awc_plan* P, int64_t nsteps, int64_t nsave, double* o
   if (count > 0 && !out) return set_err(&C->err, AWC_ERR_INVALID, "out is NULL");
   CUDA_TRY(&C->err, cudaSetDevice(C->device));
   int rc;
-  const bool loop = use_loop(P, nsave);
-  if ((rc = prepare_launch(P)) || (loop && (rc = prepare_launch(P, true)))) return rc;
+  bool loop = use_loop(P, nsave);
+  if ((rc = prepare_launch(P))) return rc;
+  if (loop && (rc = prepare_launch(P, true))) {
+    if (rc != AWC_ERR_OOM) return rc;
+    loop = false;
+  }
   // two device staging slots of N doubles: the unpitched copy of snapshot k
   // goes to slot k % 2, then to the host on the second stream while the next
   // steps run
@@ -2062,8 +2091,12 @@ int awc_plan_run_snapshots(awc_plan* P, int64_t nsteps, int64_t nsave, double* o
   const int blocks = grid_for(C, P->N, 256);
   while (it < last) {
     const int64_t next = std::min<int64_t>(last, (it / nsave + 1) * nsave);
-    rc = loop && next - it >= awc::kLoopMinSteps ? loop_range(P, it, next - it, stt, C->stream)
-                                                 : launch_range(P, it, next - it, stt, C->stream);
+    rc = awc::kLoopRefused;
+    if (loop && next - it >= awc::kLoopMinSteps) {
+      rc = loop_range(P, it, next - it, stt, C->stream);
+      loop = rc != awc::kLoopRefused;
+    }
+    if (rc == awc::kLoopRefused) rc = launch_range(P, it, next - it, stt, C->stream);
     if (rc) {
       cleanup();
       return rc;

@@ -75,6 +75,7 @@ struct awc_batch {
   // a launch shape of the per-step kernels was chosen
   awc::Loop2D loop;
   bool use_loop = true, loop_ready = false;
+  int loop_blocks = 0;  // the context's when loop_ready was set
   awc::LoopWait wait;
   std::vector<std::vector<int32_t>> h_rec_off, h_rec_ids;  // receiver groups per shot
   double* staging = nullptr;  // inside the arena (read-out)
@@ -418,6 +419,10 @@ std::vector<awc::LoopShotHost> loop_shots(const awc_batch* B) {
 
 // Whether a run of n steps goes through the on-chip loop.
 bool loop_run(awc_batch* B, int64_t n) {
+  if (B->loop_blocks != B->ctx->loop_blocks) {
+    B->loop_blocks = B->ctx->loop_blocks;
+    B->loop_ready = false;
+  }
   return B->use_loop && n >= awc::kLoopMinSteps &&
          (B->loop_ready || B->loop.fits(B->ctx, B->prec == AWC_F64, loop_shots(B)));
 }
@@ -721,10 +726,15 @@ int awc_batch_run(awc_batch* B, int64_t nsteps, int32_t use_graph, float* ms) {
   if (ms) *ms = 0.f;
   if (n <= 0) return AWC_OK;
   int rc;
-  const bool loop = loop_run(B, n);  // a launch per wave: nothing to capture
-  if (loop) use_graph = 0;
-  if ((rc = loop ? prepare_loop(B) : ensure_layout(B))) return rc;
+  bool loop = loop_run(B, n);
+  if (loop && (rc = prepare_loop(B))) {
+    if (rc != AWC_ERR_OOM) return rc;
+    loop = false;  // no room for its tables: step by step
+  }
+  if (!loop && (rc = ensure_layout(B))) return rc;
   cudaGraphExec_t ex = nullptr;
+  const int32_t graph = use_graph;
+  if (loop) use_graph = 0;  // a launch per wave: nothing to capture
   if (use_graph) {
     const uint64_t key = (uint64_t)B->ty | ((uint64_t)B->bps << 8);
     if (key != B->graph_key) {
@@ -755,7 +765,12 @@ int awc_batch_run(awc_batch* B, int64_t nsteps, int32_t use_graph, float* ms) {
   if (use_graph) {
     BATCH_TRY(C, cudaGraphLaunch(ex, C->stream));
   } else if (loop) {
-    if ((rc = launch_batch_loop(B, B->step, n, C->stream))) return rc;
+    rc = launch_batch_loop(B, B->step, n, C->stream);
+    if (rc == awc::kLoopRefused) {
+      B->loop_ready = false;
+      return awc_batch_run(B, nsteps, graph, ms);  // step by step
+    }
+    if (rc) return rc;
   } else if ((rc = launch_batch_range(B, B->step, n, C->stream))) {
     return rc;
   }
@@ -831,6 +846,7 @@ int awc_batch_autotune(awc_batch* B, int64_t steps, float* best_ms_per_step) {
       if ((rc = awc_batch_reset(B)) || (rc = awc_batch_run(B, nl, 0, &ms))) return rc;
       loop_per = std::min(loop_per, ms / (float)nl);
     }
+  if (!loop_run(B, nl)) loop_per = 1e30f;  // refused: those were the step kernels
   B->use_loop = false;
   auto trial = [&](int32_t ty, int32_t bps, float* per) -> int {
     B->ty = ty;

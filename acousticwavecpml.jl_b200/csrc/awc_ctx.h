@@ -16,6 +16,7 @@ struct awc_plan;
 struct awc_ctx {
   int device = 0;
   int num_sms = 0;
+  int loop_blocks = 0;  // most blocks of an on-chip loop's launch (num_sms unless set)
   cudaStream_t stream = nullptr;
   cudaStream_t stream2 = nullptr;  // second branch of a 3D step (the band kernel)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;

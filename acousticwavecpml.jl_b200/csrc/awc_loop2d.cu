@@ -269,7 +269,8 @@ std::vector<Loop2D::Tiling> Loop2D::tilings(const Shape& s, bool f64, int max_ti
 // tilings allow, then every wave's shots get the tile counts that minimise
 // its slowest shot's step.
 bool Loop2D::plan_waves(const awc_ctx* C) {
-  const int S = C->num_sms, ns = (int)shapes_.size(), V = f64_ ? 2 : 4;
+  const int S = C->loop_blocks, ns = (int)shapes_.size(), V = f64_ ? 2 : 4;
+  if (S < 1) return false;
   for (const Shape& sh : shapes_) {
     // a quick bound before the search: every block's threads and rows
     if (!bands_apart(sh.nx, sh.halo, sh.active[0]) || !bands_apart(sh.ny, sh.halo, sh.active[1]) ||
@@ -334,6 +335,15 @@ bool Loop2D::plan_waves(const awc_ctx* C) {
     }
     waves_.push_back(std::move(w));
   }
+  // the wave of the most tiles first: what the device has no room for is refused
+  // before anything ran
+  auto tiles = [](const Wave& w) {
+    int n = 0;
+    for (const Tiling& t : w.tiling) n += t.tiles();
+    return n;
+  };
+  std::stable_sort(waves_.begin(), waves_.end(),
+                   [&](const Wave& a, const Wave& b) { return tiles(a) > tiles(b); });
   return true;
 }
 
@@ -560,10 +570,12 @@ bool Loop2D::fits(const awc_ctx* C, bool f64, const std::vector<LoopShotHost>& s
   for (const LoopShotHost& s : shots)
     shapes.push_back(Shape{s.nx, s.ny, s.halo,
                            {{s.active[0][0], s.active[0][1]}, {s.active[1][0], s.active[1][1]}}});
-  if (planned_ && f64 == f64_ && shapes == shapes_) return !waves_.empty();
+  if (planned_ && f64 == f64_ && blocks_ == C->loop_blocks && shapes == shapes_)
+    return !waves_.empty();
   planned_ = true;
   laid_out_ = false;
   f64_ = f64;
+  blocks_ = C->loop_blocks;
   shapes_ = std::move(shapes);
   waves_.clear();
   if (!plan_waves(C)) waves_.clear();
@@ -618,8 +630,15 @@ int Loop2D::launch(awc_ctx* C, const LoopSpan& span, cudaStream_t st) {
     tag_ += (uint32_t)span.n;
     const void* k = loop_kernel<T>(wv.R);
     void* args[] = {&Q};
-    LOOP_TRY(C, cudaLaunchCooperativeKernel(k, dim3((unsigned)wv.ntiles), dim3((unsigned)wv.threads),
-                                            args, (size_t)wv.smem, st));
+    const cudaError_t e = cudaLaunchCooperativeKernel(k, dim3((unsigned)wv.ntiles), dim3((unsigned)wv.threads),
+                                                      args, (size_t)wv.smem, st);
+    if (&wv == &waves_.front() &&
+        (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported)) {
+      cudaGetLastError();
+      waves_.clear();
+      return kLoopRefused;
+    }
+    LOOP_TRY(C, e);
   }
   return AWC_OK;
 }

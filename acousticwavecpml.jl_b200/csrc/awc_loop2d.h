@@ -64,7 +64,8 @@ class Loop2D {
   bool fits(const awc_ctx* C, bool f64, const std::vector<LoopShotHost>& shots);
   // Device tables of the tiling (when it changed) and the shots' lists.
   int prepare(awc_ctx* C, bool f64, const std::vector<LoopShotHost>& shots, int32_t* err_flag);
-  // Enqueues n steps of every shot on st.
+  // Enqueues n steps of every shot on st. kLoopRefused: the device had no room for
+  // all blocks of a launch at once; nothing ran, and fits() is false from now on.
   int run(awc_ctx* C, const LoopSpan& span, cudaStream_t st);
   int64_t launches() const { return (int64_t)waves_.size(); }
 
@@ -96,6 +97,7 @@ class Loop2D {
   bool plan_waves(const awc_ctx* C);
 
   bool f64_ = false, planned_ = false, laid_out_ = false;
+  int blocks_ = 0;  // most blocks of a launch the tiling was made for
   std::vector<Shape> shapes_;
   std::vector<Wave> waves_;
   std::vector<LoopTile> tiles_;               // without the shots' lists
@@ -113,5 +115,7 @@ class Loop2D {
 // Runs shorter than this use the per-step kernels: a loop launch loads and
 // stores the whole state, which costs about as much as a few steps.
 constexpr int64_t kLoopMinSteps = 8;
+// What Loop2D::run returns beside the library's status codes.
+constexpr int kLoopRefused = 1;
 
 }  // namespace awc

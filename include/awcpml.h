@@ -107,6 +107,12 @@ void* awc_ctx_stream(const awc_ctx* ctx);
  * it. Default 40. The choice is cached with the plan. */
 int awc_ctx_set_autotune(awc_ctx* ctx, int64_t steps);
 
+/* Most blocks, one per SM, that a launch of the on-chip 2D loop may have: 0 turns
+ * the loop off, -1 (the default) is every SM of the device. A launch whose blocks
+ * the device cannot hold all at once is refused by the runtime before it starts,
+ * and the run goes through the step kernels. Results do not depend on it. */
+int awc_ctx_set_loop_blocks(awc_ctx* ctx, int32_t blocks);
+
 /* The forward solve (the time loop of acoustic_3D_xPU.jl:392-409 and the
  * returns at :541-544; 2D acoustic_2D_xPU.jl:327-343, :441-444).
  *   vel      [nx*ny*nz]       velocity [m/s]; fact = dt^2 vel^2 is formed on
