@@ -828,9 +828,9 @@ int awc_batch_field(awc_batch* B, int32_t shot, double* out) {
   return AWC_OK;
 }
 
-int awc_batch_autotune(awc_batch* B, int64_t steps, float* best_ms_per_step) {
-  if (!B) return awc::fail(nullptr, AWC_ERR_INVALID, "batch is NULL");
-  if (steps < 1) return awc::fail(B->ctx, AWC_ERR_INVALID, "steps must be >= 1");
+namespace {
+// Leaves the chosen launch in the batch; on an error whatever was tried last.
+int tune_batch(awc_batch* B, int64_t steps, float* best_ms_per_step) {
   int64_t n = std::min<int64_t>(steps, B->nt);
   float best = 1e30f;
   int32_t wty = B->ty, wbps = B->bps;
@@ -885,6 +885,21 @@ int awc_batch_autotune(awc_batch* B, int64_t steps, float* best_ms_per_step) {
   B->use_loop = loop_per < best;
   if (best_ms_per_step) *best_ms_per_step = std::min(best, loop_per);
   return awc_batch_reset(B);
+}
+}  // namespace
+
+int awc_batch_autotune(awc_batch* B, int64_t steps, float* best_ms_per_step) {
+  if (!B) return awc::fail(nullptr, AWC_ERR_INVALID, "batch is NULL");
+  if (steps < 1) return awc::fail(B->ctx, AWC_ERR_INVALID, "steps must be >= 1");
+  const int32_t ty = B->ty, bps = B->bps;
+  const bool use_loop = B->use_loop;
+  const int rc = tune_batch(B, steps, best_ms_per_step);
+  if (rc) {  // as it was
+    B->ty = ty;
+    B->bps = bps;
+    B->use_loop = use_loop;
+  }
+  return rc;
 }
 
 int awc_forward_batch(awc_ctx* C, int32_t nmodels, const awc_problem* models,

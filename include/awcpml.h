@@ -292,7 +292,8 @@ int awc_batch_get_launch(const awc_batch* batch, int32_t* tile_y, int32_t* block
  * step kernels; -1 on a bad argument. */
 int64_t awc_batch_launch_count(const awc_batch* batch, int64_t nsteps);
 /* Times the on-chip loop and every launch shape of the step kernels on the
- * batch's data, keeps the fastest, resets. */
+ * batch's data, keeps the fastest (the loop too, after awc_batch_set_launch), resets.
+ * On an error the launch is what it was. */
 int awc_batch_autotune(awc_batch* batch, int64_t steps, float* best_ms_per_step);
 /* create + autotune (nt >= 100) + run(nt) + every shot's traces + destroy;
  * traces[s] is shot s's (nt x nrec) output. */

@@ -51,8 +51,16 @@ def test_batch_timeout_and_recovery(pkg, ctx):
     with pytest.raises(pkg.AwcError) as ei:
         batch.run()
     assert ei.value.code == pkg._lib.AWC_ERR_TIMEOUT
+    # a failed autotune leaves the launch that was chosen before it
+    batch.reset()
+    batch.set_launch(16, 4)
+    with pytest.raises(pkg.AwcError):
+        batch.autotune(8)
     batch.set_wait()
     batch.reset()
+    assert batch.get_launch() == (16, 4) and batch.launch_count() == loop2d.NT
+    batch.autotune(8)
+    assert batch.launch_count() in (1, loop2d.NT)
     batch.run()
     for k in (0, 1):
         np.testing.assert_array_equal(batch.traces(k), want[k])
