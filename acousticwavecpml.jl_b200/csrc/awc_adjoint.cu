@@ -1032,13 +1032,6 @@ Groups group_nodes(const awc_problem* p, int64_t px, const int64_t* pos, int64_t
   return G;
 }
 
-// The adjoint's core box (nodes farther than one node from every active
-// band) and the shell boxes around it. Per axis the interior splits into the
-// left zone [1, h+1] (when the left side is active), the right zone
-// [n-h-2, n-2] (when the right one is) and the core range between them; the
-// shell is every product of zones but the core's (26 boxes in 3D, 8 in 2D),
-// each with its zone code as kind. When the zones of an axis leave no core
-// node between them, one generic box holds the whole interior.
 // Block ranges of A's boxes, columns of `step` nodes.
 template <typename T>
 void adj_blocks(awc::AdjStep<T>& A, int step) {
@@ -1077,8 +1070,15 @@ void adj_split(awc::AdjStep<T>& A, awc::AdjStep<T>& Z) {
   adj_blocks(Z, 2);
 }
 
+// The 3D adjoint's core box (nodes farther than one node from every active
+// band) and the shell boxes around it. Per axis the interior splits into the
+// left zone [1, h+1] (when the left side is active), the right zone
+// [n-h-2, n-2] (when the right one is) and the core range between them; the
+// shell is every product of zones but the core's (26 boxes), each with its zone
+// code as kind. When the zones of an axis leave no core node between them, one
+// generic box holds the whole interior.
 template <typename T>
-void adj_regions(awc::AdjStep<T>& A, int ndim) {
+void adj_regions(awc::AdjStep<T>& A) {
   const int64_t n[3] = {A.nx, A.ny, A.nz}, h = A.halo;
   int64_t lo[3][3], hi[3][3];  // [axis][zone]: 0 core, 1 left, 2 right
   bool split = true;
@@ -1086,10 +1086,6 @@ void adj_regions(awc::AdjStep<T>& A, int ndim) {
     for (int z = 1; z < 3; ++z) {
       lo[a][z] = 1;
       hi[a][z] = 0;  // empty
-    }
-    if (a >= ndim) {
-      lo[a][0] = hi[a][0] = 0;
-      continue;
     }
     lo[a][0] = 1;
     hi[a][0] = n[a] - 2;
@@ -1112,7 +1108,7 @@ void adj_regions(awc::AdjStep<T>& A, int ndim) {
   };
   if (!split) {
     A.core = awc::Box{1, 0, 1, 0, 0, 0, 0};  // none
-    for (int a = 0; a < ndim; ++a) {
+    for (int a = 0; a < 3; ++a) {
       lo[a][0] = 1;
       hi[a][0] = n[a] - 2;
     }
@@ -1120,7 +1116,7 @@ void adj_regions(awc::AdjStep<T>& A, int ndim) {
   } else {
     A.core = awc::Box{(int32_t)lo[0][0], (int32_t)hi[0][0], (int32_t)lo[1][0],
                       (int32_t)hi[1][0], (int32_t)lo[2][0], (int32_t)hi[2][0], 0};
-    for (int zz = 0; zz < (ndim == 3 ? 3 : 1); ++zz)
+    for (int zz = 0; zz < 3; ++zz)
       for (int zy = 0; zy < 3; ++zy)
         for (int zx = 0; zx < 3; ++zx)
           if (zx || zy || zz) add(zx, zy, zz, zx + 3 * zy + 9 * zz);
@@ -1304,20 +1300,22 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
   const Groups RG = group_nodes(p, V.px, posrecs, nrec, nullptr);
   std::vector<int64_t> snode;
   group_nodes(p, V.px, possrcs, nsrc, &snode);
-  int64_t* rnode_d;
-  int32_t *roff_d, *rids_d;
-  int64_t* snode_d;
-  ADJ_TRY(C, mem.get(&rnode_d, RG.node.size() * 8));
-  ADJ_TRY(C, mem.get(&roff_d, RG.off.size() * 4));
-  ADJ_TRY(C, mem.get(&rids_d, RG.ids.size() * 4));
-  ADJ_TRY(C, mem.get(&snode_d, snode.size() * 8));
-  if (!RG.node.empty()) {
-    ADJ_TRY(C, cudaMemcpyAsync(rnode_d, RG.node.data(), RG.node.size() * 8, cudaMemcpyHostToDevice, st));
-    ADJ_TRY(C, cudaMemcpyAsync(rids_d, RG.ids.data(), RG.ids.size() * 4, cudaMemcpyHostToDevice, st));
+  // 3D: their lists for adj_io (2D: see AdjIo2 below)
+  int64_t *rnode_d = nullptr, *snode_d = nullptr;
+  int32_t *roff_d = nullptr, *rids_d = nullptr;
+  if (p->ndim == 3) {
+    ADJ_TRY(C, mem.get(&rnode_d, RG.node.size() * 8));
+    ADJ_TRY(C, mem.get(&roff_d, RG.off.size() * 4));
+    ADJ_TRY(C, mem.get(&rids_d, RG.ids.size() * 4));
+    ADJ_TRY(C, mem.get(&snode_d, snode.size() * 8));
+    if (!RG.node.empty()) {
+      ADJ_TRY(C, cudaMemcpyAsync(rnode_d, RG.node.data(), RG.node.size() * 8, cudaMemcpyHostToDevice, st));
+      ADJ_TRY(C, cudaMemcpyAsync(rids_d, RG.ids.data(), RG.ids.size() * 4, cudaMemcpyHostToDevice, st));
+    }
+    ADJ_TRY(C, cudaMemcpyAsync(roff_d, RG.off.data(), RG.off.size() * 4, cudaMemcpyHostToDevice, st));
+    if (!snode.empty())
+      ADJ_TRY(C, cudaMemcpyAsync(snode_d, snode.data(), snode.size() * 8, cudaMemcpyHostToDevice, st));
   }
-  ADJ_TRY(C, cudaMemcpyAsync(roff_d, RG.off.data(), RG.off.size() * 4, cudaMemcpyHostToDevice, st));
-  if (!snode.empty())
-    ADJ_TRY(C, cudaMemcpyAsync(snode_d, snode.data(), snode.size() * 8, cudaMemcpyHostToDevice, st));
   // which sources sit in an active CPML band (their bracket uses S_t)
   std::vector<int8_t> sband(std::max<int64_t>(nsrc, 1), 0);
   {
@@ -1424,10 +1422,12 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
       A.off[a][s] = s == 0 ? 0 : (int32_t)(n3[a] - h - 2);
     }
   }
-  adj_regions(A, p->ndim);
   awc::AdjStep<T> Z{};  // the shell boxes the pair kernel takes
-  adj_split(A, Z);
-  const bool has_core = A.core.x0 <= A.core.x1;
+  if (p->ndim == 3) {
+    adj_regions(A);
+    adj_split(A, Z);
+  }
+  const bool has_core = p->ndim == 3 && A.core.x0 <= A.core.x1;
   const dim3 core_grid((unsigned)((A.core.x1 - A.core.x0 + 32) / 32),
                        (unsigned)((A.core.y1 - A.core.y0 + 8) / 8),
                        (unsigned)(A.core.z1 - A.core.z0 + 1));

@@ -11,8 +11,9 @@
 // library, from module load until process exit. The caller passes host
 // inputs and outputs exactly as for awc_forward.
 //
-// The solve is the same as awc_forward's FP32 2D path: the same step2d
-// kernel over a dense (unpitched) layout, with sources and receivers applied
+// The solve computes what awc_forward does in FP32 2D, step by step: the step2d
+// kernel (awc_forward's own where neither the on-chip loop nor the strips take
+// the run) over a dense (unpitched) layout, with sources and receivers applied
 // by a one-block kernel after each step.
 #include <cuda_runtime.h>
 
