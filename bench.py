@@ -255,6 +255,20 @@ def run_reference(args):
     print(json.dumps(line), flush=True)
 
 
+def batch_roofline(loop, achieved, peak):
+    """The batch leg's roofline entry. The on-chip loop is bound by instruction
+    issue, for which there is no measured peak: no fraction of one."""
+    if loop:
+        return {"bound": "issue", "achieved": achieved, "peak": None, "unit": "GB/s", "frac": None,
+                "per_launch": "all steps of one wave of shots, whose fields stay on the chip: "
+                              "achieved is A_eff of a step of every shot over its time, not "
+                              "memory traffic"}
+    return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+            "frac": achieved / peak,
+            "per_launch": "one time step of every shot of the rank's batch = one persistent "
+                          "batched-step launch; A_eff summed over shots, FP32 words"}
+
+
 def batch_leg(pkg, ctx, args, rank, world, timed, peak, keep=None):
     """Batched 2D shots, FP32: the 96 shots of the six-model layered workload,
     rank r taking shots r, r + N, ... (no data-path collective). One step of
@@ -306,14 +320,7 @@ def batch_leg(pkg, ctx, args, rank, world, timed, peak, keep=None):
             "nt": nt, "dtype": "f32", "value": len(shots) / (ms / 1e3 / k), "unit": "shots/s",
             "us_per_timestep": t_ts * 1e6, "gnodes_per_s": world * nodes / t_ts / 1e9,
             "t_eff_gbs": world * achieved,
-            "roofline": {"bound": "issue" if loop else "hbm", "achieved": achieved, "peak": peak,
-                         "unit": "GB/s", "frac": achieved / peak,
-                         "per_launch": ("all steps of one wave of shots, whose fields stay on the "
-                                        "chip: achieved is A_eff of a step of every shot over "
-                                        "its time, not memory traffic" if loop else
-                                        "one time step of every shot of the rank's batch = one "
-                                        "persistent batched-step launch; A_eff summed over "
-                                        "shots, FP32 words")},
+            "roofline": batch_roofline(loop, achieved, peak),
             "dram_roofline": dram,
             "l2": ({"traffic_bytes_per_step": l2_bytes, "achieved_gbs": l2_bytes / t_ts / 1e9,
                     "note": "ncu lts__t_bytes of one step (profiles/) over the measured step "
