@@ -1295,7 +1295,11 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
   ADJ_TRY(C, mem.get(&stf_d, srows.size() * sizeof(T)));
   ADJ_TRY(C, cudaMemcpyAsync(stf_d, srows.data(), srows.size() * sizeof(T), cudaMemcpyHostToDevice, st));
   T* sout_d = nullptr;
-  if (src_out) ADJ_TRY(C, mem.get(&sout_d, std::max<int64_t>(nt * nsrc, 1) * sizeof(T)));
+  if (src_out) {
+    ADJ_TRY(C, mem.get(&sout_d, std::max<int64_t>(nt * nsrc, 1) * sizeof(T)));
+    // sources on the rim have no adjoint: zero, which no step writes
+    ADJ_TRY(C, cudaMemsetAsync(sout_d, 0, std::max<int64_t>(nt * nsrc, 1) * sizeof(T), st));
+  }
   // receiver groups and source nodes (interior only)
   const Groups RG = group_nodes(p, V.px, posrecs, nrec, nullptr);
   std::vector<int64_t> snode;
