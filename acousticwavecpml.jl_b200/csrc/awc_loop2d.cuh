@@ -8,10 +8,12 @@
 // per tile and per SM; a block keeps its tile's p_t and p_{t-1} (in place of
 // which p_{t+1} is written) in shared memory, its fact values in registers and
 // the ψ/ξ of its CPML nodes in shared memory, and steps nt times: 1.8, 2.3 and
-// 4.7 us per step on the same grids. What bounds it: on small tiles the edges'
-// trip through L2 (0.8 us), on full ones the issue of the update (1.7 us per
-// 16384 FP32 nodes and SM) and, on the tiles of the CPML bands, the rounds of
-// band vectors that the block's threads take after it.
+// 4.7 us per step on the same grids. What bounds it is the chain of a step, with
+// at most 16 warps per SM to hide it: issue slots are 16, 37 and 31 % used on the
+// three grids, and of the warps' stalls 57, 25 and 22 % are at the block's
+// barriers (on small tiles behind the edges' trip through L2, 0.8 us; on full
+// ones behind the rounds of band vectors, which the block's threads take after
+// the update), 7, 21 and 20 % on shared memory.
 // Only the tile's edge nodes leave the SM: after each step they go to the
 // neighbour tiles' mailboxes in global memory (L2), every 32-bit word of a
 // value paired with the step's tag in one 64-bit store, so the receiver polls

@@ -256,10 +256,10 @@ def run_reference(args):
 
 
 def batch_roofline(loop, achieved, peak):
-    """The batch leg's roofline entry. The on-chip loop is bound by instruction
-    issue, for which there is no measured peak: no fraction of one."""
+    """The batch leg's roofline entry. The on-chip loop is bound by the chain of a
+    step (barriers, shared memory, edge trips), which has no peak: no fraction."""
     if loop:
-        return {"bound": "issue", "achieved": achieved, "peak": None, "unit": "GB/s", "frac": None,
+        return {"bound": "latency", "achieved": achieved, "peak": None, "unit": "GB/s", "frac": None,
                 "per_launch": "all steps of one wave of shots, whose fields stay on the chip: "
                               "achieved is A_eff of a step of every shot over its time, not "
                               "memory traffic"}
