@@ -923,7 +923,9 @@ namespace {
 struct DevMem {
   std::vector<std::pair<void*, size_t>> blocks;
   size_t next = 0;
-  void* sum = nullptr;  // the multi-shot gradient sum, outside the per-call blocks
+  // the multi-shot gradient sum or a single shot's gradient without padding,
+  // outside the per-call blocks: the two kinds of call share the blocks
+  void* sum = nullptr;
   size_t sum_bytes = 0;
   size_t refused = SIZE_MAX;  // the smallest arena of whole runs that was not to be had
   void begin() { next = 0; }
@@ -1463,7 +1465,7 @@ int adjoint_impl(awc_ctx* C, awc_plan* plan, const awc_problem* p, const double*
   // what the outputs need, ahead of the arena below, which takes what it can get
   const int64_t N = p->nx * p->ny * V.nz;
   double *dense = nullptr, *sd = nullptr;
-  if (grad_out) ADJ_TRY(C, mem.get(&dense, N * sizeof(double)));
+  if (grad_out) ADJ_TRY(C, mem.get_sum(&dense, N * sizeof(double)));
   if (src_out && nsrc > 0) ADJ_TRY(C, mem.get(&sd, nt * nsrc * sizeof(double)));
   // Checkpoints and segment fields (gradient only)
   int64_t band_elems = 0;

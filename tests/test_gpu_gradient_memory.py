@@ -96,3 +96,18 @@ def test_plans_and_batches_get_the_memory_back(pkg):
         del hold
         torch.cuda.empty_cache()
     ctx.close()
+
+
+def test_single_and_multi_shot_calls_share_their_memory(pkg):
+    s, obs = _setup(pkg)
+    ctx = pkg.Context(0)
+    ctx.set_autotune(0)
+    J, grad = pkg.adjoint.misfit_gradient_shots([s], [obs], EVERY, ctx)
+    free = _free()
+    for _ in range(2):
+        one = pkg.adjoint.misfit_gradient(s, obs, EVERY, ctx)
+        assert _free() == free and one[0] == J
+        np.testing.assert_array_equal(one[1], grad)
+        pkg.adjoint.misfit_gradient_shots([s], [obs], EVERY, ctx)
+        assert _free() == free
+    ctx.close()
