@@ -1185,7 +1185,7 @@ int64_t arena_bytes(int64_t nt, int64_t k, int64_t field, int64_t state, int64_t
 // device: memory that buys the recompute, a quarter more steps in the
 // backward pass, beside which the adjoint's kernels slow down. 232 x 212 x 232,
 // FP32, 150 steps by 50, two shots: 95.9 to 79.2 ms (7.1 GB for 5.2 GB). A longer
-// run by the same interval keeps to its segments (from about 180 steps on there).
+// run by the same interval keeps to its segments (from 175 steps on there).
 // `limit` (awc_ctx_set_keep_limit): the most bytes beyond the segments' arena, or
 // negative. A sixteenth of the device stays free beside an arena that is not held
 // yet, and what could not be had is not asked for again.

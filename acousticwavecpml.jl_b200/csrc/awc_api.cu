@@ -736,10 +736,11 @@ void kernel_params(const awc_plan* P, int which, awc::StepParams<T>& S) {
 
 // Bytes of one field on the band nodes, per SM, from which the band kernel
 // pairs the nodes of its y and z slabs: below it one node per thread keeps more
-// warps in flight. Autotuned us per step without and with pairs, n^3 grids: FP32
-// 130: 17.9, 20.9; 150: 27.0, 27.8; 175: 42.7, 42.4; 200: 60.2, 57.0; 232: 83.1,
-// 78.2; FP64 101: 18.4, 19.6; 130: 45.8, 40.6; 170: 83.9, 71.9. The line lies
-// between 150 and 175 in FP32, 101 and 130 in FP64.
+// warps in flight. Autotuned us per step without and with pairs (KB of band field
+// per SM): FP32 130^3, halo 20 (34) 17.5, 19.6; 150^3 (47) 23.6, 25.3; 175^3 (67)
+// 39.3, 39.7; 200^3 60.2, 57.0; 232^3 83.1, 78.2; FP64 101^3 (38) 17.3, 17.7; 170^3
+// 83.9, 71.9. One line for both precisions, at FP32's crossing; in FP64 pairs gain
+// from about 50 on (115^3 (51) 26.9, 25.0; 130^3 (68) 41.6, 37.1).
 constexpr int64_t BAND_WIDE_BYTES = 72000;
 
 // Splits the interior of a 3D grid into the core box (nodes outside every
