@@ -61,9 +61,9 @@ class Batch:
         return len(self.shot_nrec)
 
     def close(self):
-        if self._h:
+        if self._h and self.ctx.handle:  # see Plan.close
             _lib.lib().awc_batch_destroy(self._h)
-            self._h = ctypes.c_void_p()
+        self._h = ctypes.c_void_p()
 
     def __del__(self):
         try:

@@ -134,9 +134,11 @@ class Plan:
         self._keep = None
 
     def close(self):
-        if self._h:
+        # a context that went first (both in a collected cycle) took the stream and
+        # the rest of its state with it: there is nothing left to destroy a plan by
+        if self._h and self.ctx.handle:
             _lib.lib().awc_plan_destroy(self._h)
-            self._h = ctypes.c_void_p()
+        self._h = ctypes.c_void_p()
 
     def __del__(self):
         try:
